@@ -21,6 +21,8 @@
 // float64 atomics.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "pk_common.cuh"
 
 namespace pyl {
@@ -770,14 +772,17 @@ __global__ void __launch_bounds__(256, INTER ? 3 : 4) pk_bin_sym_kernel(BinArgs 
     }
 }
 
-// Per-CTA partial sums of pk_bin_seq_kernel into the float64 sums.  3D slots:
-// blockIdx.y splits the CTAs into groups, each thread sums one slot over its
-// group in float64.  k_per slots (axes 0/1): each CTA's plane fixes k_par, so a
-// thread per (CTA, k_per) adds its value where it belongs.
-// With items, blockIdx.z is the item: its sums, and its n_cta x stride slice of part.
-__global__ void __launch_bounds__(256) pk_part_reduce_kernel(const float *__restrict__ part, int n_cta,
-                                                             int stride, int per_group, int chunks, int axis,
-                                                             PkDims d, double *__restrict__ sums,
+// Per-CTA partial sums of the one-field kernels into the float64 sums; blockIdx.z: the
+// item of a batch.  3D slots: the first gridDim.x - per_blocks CTAs, blockIdx.y
+// splitting the slices into groups, each thread one slot of its group in float64.
+// k_per slots (axes 0/1): the chunks of a plane are all that adds to its k_par, so a
+// thread per (plane, slot) sums them and stores.  Bound by latency: a thread per slot
+// and sixteenth of the slices, with an atomic per slice and k_per slot, took 17.8 us
+// after the 11 us binning of a 128^3 field and 196 us of a batch of 24 realizations up
+// to 256^3; slices in groups of eight or more take 4.1 and 67 us.
+__global__ void __launch_bounds__(128) pk_part_reduce_kernel(const float *__restrict__ part, int n_cta, int stride,
+                                                             int chunks, int per_blocks, PkDims d,
+                                                             double *__restrict__ sums,
                                                              const pyl_pk_item *__restrict__ items)
 {
     if (items) {
@@ -786,25 +791,31 @@ __global__ void __launch_bounds__(256) pk_part_reduce_kernel(const float *__rest
     }
     double *P3 = sums, *PH = P3 + (long long)d.nb3 * 3;
     double *P2 = PH + d.nb3 + d.nb1;
-    const int n3 = d.nb3 * 4;
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    const int c0 = blockIdx.y * per_group, c1 = min(n_cta, c0 + per_group);
-    if (s < n3) {
+    const int n3 = d.nb3 * 4, blocks3 = (int)gridDim.x - per_blocks;
+    if ((int)blockIdx.x < blocks3) {
+        const int s = blockIdx.x * blockDim.x + threadIdx.x;
+        if (s >= n3) return;
+        const int per_group = (n_cta + (int)gridDim.y - 1) / (int)gridDim.y;
+        const int c0 = blockIdx.y * per_group, c1 = min(n_cta, c0 + per_group);
         double acc = 0.0;
+#pragma unroll 8
         for (int c = c0; c < c1; c++) acc += (double)part[(long long)c * stride + s];
         if (acc != 0.0) {
             const int bin = s >> 2, k = s & 3;
             if (k < 3) atomicAdd(P3 + (long long)bin * 3 + k, acc);
             else atomicAdd(PH + bin, acc);
         }
-    } else if (axis != 2 && s < n3 + d.kmax_per + 1) {
-        const int kper = s - n3;
-        for (int c = c0; c < c1; c++) {
-            const float v = part[(long long)c * stride + s];
-            if (v == 0.0f) continue;
-            const int kpar = c / chunks;        // pk_bin_sym_kernel: CTA c holds plane |k_par| = c / chunks
-            atomicAdd(P2 + (long long)(d.kmax_par + 1) * kper + kpar, (double)v);
-        }
+        return;
+    }
+    const int slots = d.kmax_per + 1, planes = n_cta / chunks;
+    const long long total = (long long)planes * slots, step = (long long)per_blocks * gridDim.y * blockDim.x;
+    for (long long i = ((long long)blockIdx.y * per_blocks + (blockIdx.x - blocks3)) * blockDim.x + threadIdx.x;
+         i < total; i += step) {
+        const int plane = (int)(i / slots), kper = (int)(i % slots);
+        const float *src = part + (long long)plane * chunks * stride + n3 + kper;
+        double acc = 0.0;
+        for (int c = 0; c < chunks; c++) acc += (double)src[(long long)c * stride];
+        P2[(long long)(d.kmax_par + 1) * kper + plane] = acc;
     }
 }
 
@@ -812,7 +823,9 @@ __global__ void __launch_bounds__(256) pk_part_reduce_kernel(const float *__rest
 __global__ void __launch_bounds__(256) pk_items_zero_kernel(const pyl_pk_item *__restrict__ items, long long len)
 {
     double *s = items[blockIdx.x].sums;
-    for (long long i = threadIdx.x; i < len; i += blockDim.x) s[i] = 0.0;
+    for (long long i = blockIdx.y * (long long)blockDim.x + threadIdx.x; i < len;
+         i += (long long)gridDim.y * blockDim.x)
+        s[i] = 0.0;
 }
 
 // Data-independent per-bin sums: N3 and K3 = sum |k| by 3D bin, N1 by |k_par| for
@@ -1067,6 +1080,22 @@ inline SeqPart seq_part(const PkDims &d, int axis)
     return p;
 }
 
+// Groups of eight or more slices while the launch fills the SMs; a few k_per slots
+// (planes x slots) per thread.
+int reduce_parts(const float *part, unsigned n_cta, int stride, int chunks, int axis, const PkDims &d, double *sums,
+                 const pyl_pk_item *items, int n_items, cudaStream_t st)
+{
+    const int blocks3 = (d.nb3 * 4 + 127) / 128;
+    int groups = (int)((8LL * num_sms() + blocks3 * n_items - 1) / ((long long)blocks3 * n_items));
+    groups = std::max(1, std::min(groups, (int)n_cta / 8));
+    const long long planes = (long long)sym_groups(d.dims) * (d.kmax_per + 1);
+    const int per_blocks = axis == 2 ? 0 : (int)std::max(1LL, std::min(planes / (256LL * groups), 4LL * num_sms()));
+    pk_part_reduce_kernel<<<dim3(blocks3 + per_blocks, groups, (unsigned)n_items), 128, 0, st>>>(
+        part, (int)n_cta, stride, chunks, per_blocks, d, sums, items);
+    PYL_LAUNCH_CHECK();
+    return PYL_OK;
+}
+
 }  // namespace
 }  // namespace pyl
 
@@ -1171,11 +1200,7 @@ extern "C" int pyl_pk_bin(const void *dk, const void *dk_interlaced, int n_field
 #undef PYL_SEQ
         PYL_LAUNCH_CHECK();
         if (a.part) {
-            const int slots = d.nb3 * 4 + (axis == 2 ? 0 : d.kmax_per + 1);
-            const int groups = 16, per_group = (int)((blocks + groups - 1) / groups);
-            pk_part_reduce_kernel<<<dim3((slots + 255) / 256, groups), 256, 0, st>>>(
-                a.part, (int)blocks, sp.stride, per_group, a.chunks, axis, d, sums, nullptr);
-            PYL_LAUNCH_CHECK();
+            return reduce_parts(a.part, blocks, sp.stride, a.chunks, axis, d, sums, nullptr, 1, st);
         }
         return PYL_OK;
     }
@@ -1312,7 +1337,8 @@ extern "C" int pyl_pk_bin_batch(const pyl_pk_item *items, int n_items, int dims,
     a.rows_per_cta = bp.rows_per_cta;
     a.part = (float *)((char *)workspace + ring_bytes);
     a.part_stride = bp.stride;
-    pk_items_zero_kernel<<<n_items, 256, 0, st>>>(items, pyl_pk_sums_len(dims, 1));
+    const long long len = pyl_pk_sums_len(dims, 1);
+    pk_items_zero_kernel<<<dim3((unsigned)n_items, (unsigned)std::min(16LL, (len + 1023) / 1024)), 256, 0, st>>>(items, len);
     PYL_LAUNCH_CHECK();
     PYL_CUDA(cudaMemsetAsync(a.part, 0, sizeof(float) * (size_t)bp.blocks * bp.stride * n_items, st));
     const dim3 grid(bp.blocks, (unsigned)n_items);
@@ -1332,12 +1358,7 @@ extern "C" int pyl_pk_bin_batch(const pyl_pk_item *items, int n_items, int dims,
     }
 #undef PYL_SEQB
     PYL_LAUNCH_CHECK();
-    const int slots = d.nb3 * 4 + (axis == 2 ? 0 : d.kmax_per + 1);
-    const int groups = 16, per_group = (int)((bp.blocks + groups - 1) / groups);
-    pk_part_reduce_kernel<<<dim3((slots + 255) / 256, groups, (unsigned)n_items), 256, 0, st>>>(
-        a.part, (int)bp.blocks, bp.stride, per_group, a.chunks, axis, d, nullptr, items);
-    PYL_LAUNCH_CHECK();
-    return PYL_OK;
+    return reduce_parts(a.part, bp.blocks, bp.stride, a.chunks, axis, d, nullptr, items, n_items, st);
 }
 
 extern "C" int pyl_pk_geometry(int dims, int axis, double *geom, void *workspace, size_t workspace_bytes,
