@@ -23,7 +23,7 @@
 
 #include <algorithm>
 
-#include "pk_common.cuh"
+#include "pk_rows.cuh"
 
 namespace pyl {
 namespace {
@@ -392,51 +392,13 @@ inline int seq_chunk(int nz)
 inline unsigned seq_chunk_magic(int chunk) { return (unsigned)((0x100000000ull + chunk - 1) / chunk); }
 
 
-// ---- the four sign rows of a representative (|kx|, |ky|) ----------------------------
-// Every bin index (|k|^2 = kx^2 + ky^2 + kz^2, k_per^2, k_par^2 for any line of
-// sight) and every Legendre weight depends on kx^2 and ky^2 only, so the rows
-// (+-kx, +-ky) share their bins at every kz: the one-field kernels sum the (up to
-// four) modes' |d|^2 and phase^2 at each kz and walk the bins once for all of
-// them (a quarter of the bin walk, its flushes and the staging of one row at a
-// time; the loads and per-mode arithmetic are the same).  The representatives are
-// 0..dims/2 on each axis; 0 and dims/2 have no partner.  Each mode's power is
-// |v|^2 mf^2 with mf the deconvolution factor, shared by the four modes; its phase
-// atan(Re v / |v|) does not depend on mf > 0.
-__host__ __device__ inline int sym_groups(int dims) { return dims / 2 + 1; }
-
-struct SignRows {
-    long long off[4];       // row r = (y sign << 1) | x sign
-    float2 pxy[4];          // interlacing phase exp(i pi (kx + ky) / dims) of each row
-    unsigned skip0, skipm;  // rows whose kz = 0 / kz = dims/2 modes the Hermitian skip drops
-    unsigned used;          // rows that exist (a representative without partner repeats row 0)
-};
-
-template <bool INTER>
-__device__ __forceinline__ SignRows sign_rows(int xr, int yr, const PkDims &d, const float2 *ph)
-{
-    const int dims = d.dims;
-    const bool even = (dims & 1) == 0;
-    const int nx = (xr == 0 || 2 * xr == dims) ? 1 : 2, ny = (yr == 0 || 2 * yr == dims) ? 1 : 2;
-    SignRows R;
-    R.skip0 = R.skipm = 0u;
-    R.used = 1u | (nx == 2 ? 2u : 0u) | (ny == 2 ? 4u : 0u) | (nx == 2 && ny == 2 ? 8u : 0u);
-#pragma unroll
-    for (int r = 0; r < 4; r++) {
-        const int kxx = ((r & 1) && nx == 2) ? dims - xr : xr;     // in range for every r
-        const int kyy = ((r & 2) && ny == 2) ? dims - yr : yr;
-        R.off[r] = ((long long)kxx * dims + kyy) * d.nz;
-        const int kx = freq_of(kxx, dims), ky = freq_of(kyy, dims);
-        R.pxy[r] = make_float2(1.0f, 0.0f);
-        if (INTER) {
-            const float2 px = ph[kxx], py = ph[kyy];
-            R.pxy[r] = make_float2(px.x * py.x - px.y * py.y, px.x * py.y + px.y * py.x);
-        }
-        if (hermitian_skip(kx, ky, 0, d)) R.skip0 |= 1u << r;
-        if (even && hermitian_skip(kx, ky, d.middle, d)) R.skipm |= 1u << r;
-    }
-    return R;
-}
-
+// ---- one field: the four sign rows of a representative at once (pk_rows.cuh) --------
+// The one-field kernels sum the (up to four) modes' |d|^2 and phase^2 at each kz and walk
+// the bins once for all of them (a quarter of the bin walk, its flushes and the staging
+// of one row at a time; the loads and per-mode arithmetic are the same).  Each mode's
+// power is |v|^2 mf^2 with mf the deconvolution factor, shared by the four modes; its
+// phase atan(Re v / |v|) does not depend on mf > 0.
+//
 // Pass 1 for one representative: the summed power and phase^2 of its rows at each
 // kz (lanes along kz, coalesced), into the warp's staging array at kz + kz / chunk.
 // All four rows are loaded (in range for every r), so an iteration's loads issue
