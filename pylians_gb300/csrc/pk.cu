@@ -4,52 +4,72 @@
 #include <cuda_runtime.h>
 
 #include <math.h>
+#include <algorithm>
 #include <vector>
 
-#include "pk_common.cuh"
+#include "pk_rows.cuh"
 
 namespace pyl {
 
 namespace {
 
 // Per-axis float64 tables in shared memory, built once per CTA: the MAS factor
-// C(k) = (x / sin x)^p of each frequency and, for the interlaced combine, the
-// phase e^{i pi k / N}.  Per mode: the float64 product C(kx) C(ky) C(kz) rounded to
-// float32 (Pk_library.pyx:86-87,353-355) and the phase as the product of the three
-// axis phases (equal to e^{i pi (kx+ky+kz)/N} to float64 rounding).
+// C(k) = (x / sin x)^p of each |k| and, for the interlaced combine, the phase
+// e^{i pi k / N}.  Per mode: the float64 product C(kx) C(ky) C(kz) rounded to
+// float32 (Pk_library.pyx:86-87,353-355), one for the four sign rows (+-kx, +-ky) that a
+// warp takes together, and the phase as the product of the three axis phases (equal to
+// e^{i pi (kx+ky+kz)/N} to float64 rounding).  256^3: 60 us with a mode per thread (two
+// float64 products and two 64-bit divisions each), 29 us so.
 __global__ void __launch_bounds__(256) deconvolve_kernel(float2 *dk, const float2 *dk2, PkDims d, int p)
 {
     extern __shared__ double dtab[];
     const int dims = d.dims;
-    double *corr = dtab;                        // [dims]
-    double2 *ph = (double2 *)(dtab + dims);     // [dims] when interlaced
-    for (int i = threadIdx.x; i < dims; i += blockDim.x) {
-        const int k = freq_of(i, dims);
-        corr[i] = mas_corr_d(k, dims, p);
-        if (dk2) {
+    double *corr = dtab;                        // [nz]
+    double2 *ph = (double2 *)(dtab + (d.nz + 1) / 2 * 2);   // [dims] when interlaced
+    for (int i = threadIdx.x; i < d.nz; i += blockDim.x) corr[i] = mas_corr_d(i, dims, p);
+    if (dk2)
+        for (int i = threadIdx.x; i < dims; i += blockDim.x) {
             double s, c;
-            sincospi((double)k / dims, &s, &c);
+            sincospi((double)freq_of(i, dims) / dims, &s, &c);
             ph[i] = make_double2(c, s);
         }
-    }
     __syncthreads();
-    const long long total = (long long)dims * dims * d.nz;
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
-        const int kz = (int)(i % d.nz);
-        const long long rr = i / d.nz;
-        const int kyy = (int)(rr % dims), kxx = (int)(rr / dims);
-        float2 v = dk[i];
+    const int G = sym_groups(dims), lane = threadIdx.x & 31;
+    const int nwarp = (int)(gridDim.x * (blockDim.x >> 5));
+    for (int rep = (int)(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)); rep < G * G; rep += nwarp) {
+        const int xr = rep / G, yr = rep % G;
+        const SignRows R = sign_rows<false>(xr, yr, d, nullptr);
+        const double cxy = corr[xr] * corr[yr];
+        double2 ab[4];
         if (dk2) {
-            const double2 a = ph[kxx], b = ph[kyy], e = ph[kz];
-            const double2 ab = make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
-            const float pc = (float)(ab.x * e.x - ab.y * e.y), ps = (float)(ab.x * e.y + ab.y * e.x);
-            const float2 w = dk2[i];
-            v.x = 0.5f * (v.x + (w.x * pc - w.y * ps));
-            v.y = 0.5f * (v.y + (w.x * ps + w.y * pc));
+#pragma unroll
+            for (int r = 0; r < 4; r++) {
+                const long long row = R.off[r] / d.nz;
+                const double2 a = ph[row / dims], b = ph[row % dims];
+                ab[r] = make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+            }
         }
-        const float mf = (float)(corr[kxx] * corr[kyy] * corr[kz]);
-        dk[i] = make_float2(__fmul_rn(v.x, mf), __fmul_rn(v.y, mf));
+        for (int kz = lane; kz < d.nz; kz += 32) {
+            const float mf = (float)(cxy * corr[kz]);
+            float2 v[4], w[4];
+#pragma unroll
+            for (int r = 0; r < 4; r++) {
+                if (!((R.used >> r) & 1u)) continue;
+                v[r] = dk[R.off[r] + kz];
+                if (dk2) w[r] = dk2[R.off[r] + kz];
+            }
+#pragma unroll
+            for (int r = 0; r < 4; r++) {
+                if (!((R.used >> r) & 1u)) continue;
+                if (dk2) {
+                    const double2 e = ph[kz];
+                    const float pc = (float)(ab[r].x * e.x - ab[r].y * e.y), ps = (float)(ab[r].x * e.y + ab[r].y * e.x);
+                    v[r].x = 0.5f * (v[r].x + (w[r].x * pc - w[r].y * ps));
+                    v[r].y = 0.5f * (v[r].y + (w[r].x * ps + w[r].y * pc));
+                }
+                dk[R.off[r] + kz] = make_float2(__fmul_rn(v[r].x, mf), __fmul_rn(v[r].y, mf));
+            }
+        }
     }
 }
 
@@ -130,12 +150,13 @@ extern "C" int pyl_mas_deconvolve(void *dk, const void *dk_interlaced, int dims,
     PYL_CHECK_ARG(dims >= 2 && dims <= 8192, "dims out of range");
     PYL_CHECK_ARG(mas_p >= 0 && mas_p <= 4, "MAS exponent must be 0..4");
     const PkDims d = pk_dims(dims);
-    const long long total = (long long)dims * dims * d.nz;
-    const size_t smem = sizeof(double) * (size_t)dims * (dk_interlaced ? 3 : 1);
+    const size_t smem = sizeof(double) * ((size_t)(d.nz + 1) / 2 * 2 + (dk_interlaced ? 2 * (size_t)dims : 0));
     PYL_CUDA(ensure_smem(deconvolve_kernel, smem));
-    // two CTAs per SM: each builds its tables once and strides over the modes
-    deconvolve_kernel<<<blocks_for(total, 256, 2), 256, smem, (cudaStream_t)stream>>>(
-        (float2 *)dk, (const float2 *)dk_interlaced, d, mas_p);
+    // a warp per representative; four CTAs per SM: each builds its tables once
+    const long long reps = (long long)sym_groups(dims) * sym_groups(dims);
+    const long long blocks = std::min((reps + 7) / 8, 4LL * num_sms());
+    deconvolve_kernel<<<(unsigned)blocks, 256, smem, (cudaStream_t)stream>>>((float2 *)dk, (const float2 *)dk_interlaced,
+                                                                            d, mas_p);
     PYL_LAUNCH_CHECK();
     return PYL_OK;
 }
