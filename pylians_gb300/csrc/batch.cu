@@ -11,6 +11,7 @@
 // arithmetic is the one of mas.cu (MAS_library.pyx:123-545).
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <string>
 
 #include "common.cuh"
@@ -151,10 +152,16 @@ __global__ void __launch_bounds__(256) scale_value_kernel(float *g, long long n,
 //   bt_place:   persistent over the items: per 4096-particle batch, shared-memory
 //               ranks per bin, one global atomic per bin to reserve a range,
 //               records (x, y, z, 1) written into their bins' ranges;
-//   bt_deposit: persistent over the bins: 10.22 fixed-point shared-memory
-//               accumulation of the bin (+ halo) for its realization's MAS, both
-//               grids when interlaced, red.global into the realization's grid(s)
-//               scaled to the overdensity.
+//   bt_adds, bt_parts, bt_list: the deposit's work list: every bin of every grid (the
+//               interlaced one apart), those of more than a quarter of an SM's share
+//               of all corner additions in parts of that size (BinShare), so that
+//               the crowded bins of a small grid (7.9 million particles in the 8 bins
+//               of 64^3) do not keep a few SMs busy after all others are done;
+//   bt_deposit: persistent over the parts: 10.22 fixed-point shared-memory
+//               accumulation of the bin (+ halo) for its realization's MAS,
+//               red.global into the realization's grid scaled to the overdensity.
+//               24 realizations up to 256^3: 3.0 ms with whole bins (2.3 ms of it
+//               one bin of a 64^3 grid), 1.9 ms in parts.
 constexpr int BT_MAX_TILES = 4096;        // bins per realization (dims <= 512)
 constexpr int BT_BATCH = 4096;            // placement batch (particles)
 
@@ -240,7 +247,126 @@ __global__ void __launch_bounds__(1024) bt_count_kernel(const pyl_batch_real *__
     }
 }
 
-// Exclusive scan of n counts into offsets[0..n] and cursor[0..n), one CTA.
+__host__ __device__ inline unsigned bt_corners(int mas)
+{
+    const unsigned s = mas == PYL_MAS_NGP ? 1u : (unsigned)mas;
+    return s * s * s;
+}
+
+// Parts of a batch of `adds` corner additions: at most BT_PARTS_PER_SM an SM, none below
+// PART_ADDS.
+constexpr unsigned BT_PARTS_PER_SM = 4;
+
+__device__ __forceinline__ unsigned bt_part_len(unsigned long long adds, unsigned sms, int mas)
+{
+    const unsigned long long share = adds / (BT_PARTS_PER_SM * sms);
+    return (unsigned)((share > PART_ADDS ? share : PART_ADDS) / bt_corners(mas)) + 1u;
+}
+
+// The most parts that a batch can have (its grids' bins, and the shares that all additions
+// make, rounded up), and the most bins in parts: each has more than a share of all
+// additions, and more than PART_ADDS of them, PART_ADDS / 64 particles at least.
+inline size_t bt_max_parts(unsigned total_tiles)
+{
+    return 2 * (size_t)total_tiles + (BT_PARTS_PER_SM + 1) * (size_t)num_sms();
+}
+inline size_t bt_max_shared(unsigned total_tiles, long long total_particles)
+{
+    return std::min({(size_t)BT_PARTS_PER_SM * num_sms(), 2 * (size_t)total_tiles,
+                     2 * (size_t)(total_particles / (PART_ADDS / 64))});
+}
+
+struct BtPart {
+    unsigned tile, real;
+    unsigned first, len;        // records of the bin
+    unsigned inter;             // 1: the interlaced grid
+    unsigned parts, shared;     // of the bin; with several, the index of their BinShare
+    unsigned reserved;
+};
+
+// Words of a BinShare: the largest bin (PCS, interlaced).
+constexpr size_t BT_SHARE_CELLS = FxShape<PYL_MAS_PCS, true>::CELLS;
+
+// Realization of a bin: the last one with tile_base <= t.
+__device__ __forceinline__ int bt_real_of(const unsigned *__restrict__ tile_base, int n_reals, unsigned t)
+{
+    int lo = 0, hi = n_reals;
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (tile_base[mid] <= t) lo = mid; else hi = mid;
+    }
+    return lo;
+}
+
+// Corner additions of the whole batch.
+__global__ void __launch_bounds__(256) bt_adds_kernel(const pyl_batch_real *__restrict__ reals, int n_reals,
+                                                      const unsigned *__restrict__ tile_base, unsigned total_tiles,
+                                                      const unsigned *__restrict__ counts, unsigned long long *adds)
+{
+    const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
+    unsigned long long a = 0;
+    if (t < total_tiles) {
+        const pyl_batch_real &r = reals[bt_real_of(tile_base, n_reals, t)];
+        a = (unsigned long long)counts[t] * bt_corners(r.mas) * (r.grid_interlaced ? 2u : 1u);
+    }
+    for (int o = 16; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
+    if ((threadIdx.x & 31) == 0 && a) atomicAdd(adds, a);
+}
+
+// Parts of each bin.
+__global__ void __launch_bounds__(256) bt_parts_kernel(const pyl_batch_real *__restrict__ reals, int n_reals,
+                                                       const unsigned *__restrict__ tile_base, unsigned total_tiles,
+                                                       const unsigned *__restrict__ counts,
+                                                       const unsigned long long *__restrict__ adds, unsigned sms,
+                                                       unsigned *__restrict__ parts)
+{
+    const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= total_tiles) return;
+    const pyl_batch_real &r = reals[bt_real_of(tile_base, n_reals, t)];
+    const unsigned len = bt_part_len(*adds, sms, r.mas);
+    parts[t] = (counts[t] / len + (counts[t] % len != 0u)) * (r.grid_interlaced ? 2u : 1u);
+}
+
+// The work list, in bin order: a bin's parts of the plain grid, then of the interlaced
+// one.  Each grid's bin in parts takes a BinShare.
+__global__ void __launch_bounds__(256) bt_list_kernel(const pyl_batch_real *__restrict__ reals, int n_reals,
+                                                      const unsigned *__restrict__ tile_base, unsigned total_tiles,
+                                                      const unsigned *__restrict__ counts,
+                                                      const unsigned long long *__restrict__ adds, unsigned sms,
+                                                      const unsigned *__restrict__ first_part, unsigned max_parts,
+                                                      unsigned max_shared, unsigned *shared_count,
+                                                      BtPart *__restrict__ list)
+{
+    const unsigned t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);      // a warp per bin
+    const unsigned lane = threadIdx.x & 31u;
+    if (t >= total_tiles) return;
+    const unsigned b = first_part[t], n = first_part[t + 1] - b;
+    if (n == 0u) return;
+    const int real = bt_real_of(tile_base, n_reals, t);
+    const unsigned len = bt_part_len(*adds, sms, reals[real].mas), grids = reals[real].grid_interlaced ? 2u : 1u;
+    const unsigned per_grid = n / grids;
+    unsigned shared = 0u;
+    if (per_grid > 1u) {
+        if (lane == 0u) shared = atomicAdd(shared_count, grids);
+        shared = __shfl_sync(0xffffffffu, shared, 0);
+        if (shared + grids > max_shared) return;            // not reached: see bt_max_shared
+    }
+    for (unsigned i = lane; i < n && b + i < max_parts; i += 32) {
+        const unsigned first = (i % per_grid) * len, g = i / per_grid;
+        list[b + i] = BtPart{t, (unsigned)real, first, min(len, counts[t] - first), g, per_grid, shared + g, 0u};
+    }
+}
+
+// Zeroes the words of the BinShares in use (blockIdx.y), gridDim.x CTAs each.
+__global__ void __launch_bounds__(256) bt_share_zero_kernel(const unsigned *__restrict__ shared_count,
+                                                            unsigned long long *__restrict__ share)
+{
+    if (blockIdx.y >= *shared_count) return;
+    unsigned long long *z = share + blockIdx.y * BT_SHARE_CELLS;
+    for (size_t i = blockIdx.x * blockDim.x + threadIdx.x; i < BT_SHARE_CELLS; i += gridDim.x * blockDim.x) z[i] = 0ull;
+}
+
+// Exclusive scan of n counts into offsets[0..n] and (where given) cursor[0..n), one CTA.
 __global__ void __launch_bounds__(1024) bt_scan_kernel(const unsigned *__restrict__ counts, unsigned n,
                                                        unsigned *__restrict__ offsets, unsigned *__restrict__ cursor)
 {
@@ -260,7 +386,7 @@ __global__ void __launch_bounds__(1024) bt_scan_kernel(const unsigned *__restric
     unsigned long long run = part[threadIdx.x] - sum;
     for (unsigned i = b; i < e; i++) {
         offsets[i] = (unsigned)run;
-        cursor[i] = (unsigned)run;
+        if (cursor) cursor[i] = (unsigned)run;
         run += counts[i];
     }
     if (threadIdx.x == blockDim.x - 1) offsets[n] = (unsigned)part[threadIdx.x];
@@ -387,105 +513,154 @@ __global__ void __launch_bounds__(1024) bt_place_kernel(const pyl_batch_real *__
     }
 }
 
-// Deposit of one bin of realization r (MAS, interlacing as template
-// parameters), fixed point with the float32 redo of mode 1.
+// ---- bins in parts ---------------------------------------------------------------
+// A bin whose records go to several CTAs keeps one 64-bit fixed-point word per cell in
+// global memory: every CTA adds its cells there, and the last one to arrive converts
+// the sums, so the grid gets the same value as from one CTA (integer sums do not depend
+// on the order or the grouping of the adds; 64 bits cannot wrap).
+struct BinShare {
+    unsigned long long *acc;     // the bin's words (zeroed before the launch)
+    unsigned *done;              // parts that have arrived (zeroed before the launch)
+    unsigned parts;              // of the bin; 1: acc and done are not used
+};
+
+__device__ __forceinline__ void share_add(const BinShare &sh, const unsigned *smw, int cells)
+{
+    for (int c = threadIdx.x; c < cells; c += blockDim.x) {
+        const unsigned w = smw[c];
+        if (w != 0u) atomicAdd(sh.acc + c, (unsigned long long)w);
+    }
+}
+
+// All threads, after share_add (or instead of it: a part summed in float32 goes to the
+// grid by itself): true in the CTA that arrives last, which then sees every part's words.
+__device__ __forceinline__ bool share_arrive(const BinShare &sh)
+{
+    __threadfence();
+    __syncthreads();
+    const bool last = threadIdx.x == 0 && atomicAdd(sh.done, 1u) + 1u == sh.parts;
+    const bool mine = __syncthreads_or((int)last);
+    __threadfence();
+    return mine;
+}
+
+template <int MAS>
+__device__ __forceinline__ float share_value(const BinShare &sh, int c)
+{
+    const float v = __ull2float_rn(__ldcg(sh.acc + c));
+    return MAS == PYL_MAS_NGP ? v : __fmul_rn(v, FX_INV);
+}
+
+// Deposit of the records [begin, end) of one bin of realization r onto its plain grid or
+// (PASS 1) its interlaced one; MAS and interlacing (the shape of the bin's cells) as
+// template parameters; fixed point with the float32 redo of mode 1.
 template <int MAS, bool INTER>
 __device__ __forceinline__ void bt_deposit_bin(unsigned *smw, const float4 *__restrict__ rec, unsigned begin,
-                                               unsigned end, const pyl_batch_real &r, const int *o)
+                                               unsigned end, const pyl_batch_real &r, const int *o, int pass,
+                                               const BinShare &sh)
 {
     using FS = FxShape<MAS, INTER>;
     constexpr int S = Support<MAS>::S, E = FS::E, CELLS = FS::CELLS;
     float *facc = (float *)smw;
     const long long d = r.dims;
-    for (int pass = 0; pass < (INTER ? 2 : 1); pass++) {
-        for (int mode = 0; mode < 2; mode++) {
-            uint4 *z4 = (uint4 *)smw;
-            for (int c = threadIdx.x; c < FS::SMEM / 16; c += blockDim.x) z4[c] = make_uint4(0u, 0u, 0u, 0u);
-            __syncthreads();
-            unsigned bad = 0u, seen = 0u;
-            for (unsigned i = begin + threadIdx.x; i < end; i += blockDim.x) {
-                const float4 p = rec[i];
-                float C[3][S];
-                const int b0 = pass ? fx_support<MAS, 1, E>(p, r.inv, r.halfcell, r.dims, o, C)
-                                    : fx_support<MAS, 0, E>(p, r.inv, r.halfcell, r.dims, o, C);
-                if (mode == 0) {
-                    if (MAS == PYL_MAS_CIC) bad |= (unsigned)!(C[0][1] >= 0.0f && C[1][1] >= 0.0f && C[2][1] >= 0.0f);
-                    // z weights times 2^22 (exact): each corner one FFMA into the fixed-point format
+    for (int mode = 0; mode < 2; mode++) {
+        uint4 *z4 = (uint4 *)smw;
+        for (int c = threadIdx.x; c < FS::SMEM / 16; c += blockDim.x) z4[c] = make_uint4(0u, 0u, 0u, 0u);
+        __syncthreads();
+        unsigned bad = 0u, seen = 0u;
+        for (unsigned i = begin + threadIdx.x; i < end; i += blockDim.x) {
+            const float4 p = rec[i];
+            float C[3][S];
+            const int b0 = INTER && pass ? fx_support<MAS, 1, E>(p, r.inv, r.halfcell, r.dims, o, C)
+                                         : fx_support<MAS, 0, E>(p, r.inv, r.halfcell, r.dims, o, C);
+            if (mode == 0) {
+                if (MAS == PYL_MAS_CIC) bad |= (unsigned)!(C[0][1] >= 0.0f && C[1][1] >= 0.0f && C[2][1] >= 0.0f);
+                // z weights times 2^22 (exact): each corner one FFMA into the fixed-point format
 #pragma unroll
-                    for (int q = 0; q < S; q++) C[2][q] = __fmul_rn(C[2][q], FX_SCALE);
-                    seen |= fx_scatter_or<MAS, E, (MAS == PYL_MAS_NGP), true>(smw, b0, C);
-                } else {
-                    float_scatter<MAS, E>(facc, b0, C);
-                }
+                for (int q = 0; q < S; q++) C[2][q] = __fmul_rn(C[2][q], FX_SCALE);
+                seen |= fx_scatter_or<MAS, E, (MAS == PYL_MAS_NGP), true>(smw, b0, C);
+            } else {
+                float_scatter<MAS, E>(facc, b0, C);
             }
-            if (__syncthreads_or((int)(bad | (seen >> 31))) && mode == 0) {
-                __syncthreads();
-                continue;
-            }
-            float *out = pass == 0 ? r.grid : r.grid_interlaced;
+        }
+        if (__syncthreads_or((int)(bad | (seen >> 31))) && mode == 0) {
+            __syncthreads();
+            continue;
+        }
+        float *out = INTER && pass ? r.grid_interlaced : r.grid;
+        auto add = [&](int c, float v) {
+            const int lz = c % E, ly = (c / E) % E, lx = c / (E * E);
+            const long long gx = add_wrap(o[0], lx, d), gy = add_wrap(o[1], ly, d), gz = add_wrap(o[2], lz, d);
+            atomicAdd(out + (gx * d + gy) * d + gz, __fmul_rn(v, r.scale));
+        };
+        if (sh.parts > 1 && mode == 0) {
+            share_add(sh, smw, CELLS);
+        } else {
             for (int c = threadIdx.x; c < CELLS; c += blockDim.x) {
                 const unsigned w = smw[c];
                 if (w == 0u) continue;
-                const float v = mode == 1 ? __uint_as_float(w)
-                                          : (MAS == PYL_MAS_NGP ? __uint2float_rn(w)
-                                                                : __fmul_rn(__uint2float_rn(w), FX_INV));
-                const int lz = c % E, ly = (c / E) % E, lx = c / (E * E);
-                const long long gx = add_wrap(o[0], lx, d), gy = add_wrap(o[1], ly, d), gz = add_wrap(o[2], lz, d);
-                atomicAdd(out + (gx * d + gy) * d + gz, __fmul_rn(v, r.scale));
+                add(c, mode == 1 ? __uint_as_float(w)
+                                 : (MAS == PYL_MAS_NGP ? __uint2float_rn(w) : __fmul_rn(__uint2float_rn(w), FX_INV)));
             }
-            __syncthreads();
-            break;
         }
+        if (sh.parts > 1 && share_arrive(sh))
+            for (int c = threadIdx.x; c < CELLS; c += blockDim.x) {
+                const float v = share_value<MAS>(sh, c);
+                if (v != 0.0f) add(c, v);
+            }
+        __syncthreads();
+        break;
     }
 }
 
 constexpr size_t BT_DEPOSIT_SMEM = FxShape<PYL_MAS_PCS, true>::SMEM;
 
-__global__ void __launch_bounds__(1024) bt_deposit_kernel(const pyl_batch_real *__restrict__ reals, int n_reals,
+__global__ void __launch_bounds__(1024) bt_deposit_kernel(const pyl_batch_real *__restrict__ reals,
                                                           const unsigned *__restrict__ tile_base,
-                                                          unsigned total_tiles, const unsigned *__restrict__ offsets,
-                                                          unsigned n_total, const float4 *__restrict__ rec,
-                                                          unsigned *counter)
+                                                          const BtPart *__restrict__ list,
+                                                          const unsigned *__restrict__ n_parts, unsigned max_parts,
+                                                          const unsigned *__restrict__ offsets, unsigned n_total,
+                                                          const float4 *__restrict__ rec, unsigned long long *share,
+                                                          unsigned *done, unsigned *counter)
 {
     extern __shared__ __align__(16) unsigned bsm[];
     __shared__ int cur;
+    const unsigned total = min(*n_parts, max_parts);
     for (;;) {
         if (threadIdx.x == 0) cur = (int)atomicAdd(counter, 1u);
         __syncthreads();
-        const unsigned t = (unsigned)cur;
-        if (t >= total_tiles) break;
-        const unsigned end = min(offsets[t + 1], n_total), begin = min(offsets[t], end);
-        if (begin == end) {
-            __syncthreads();
-            continue;
-        }
-        int lo = 0, hi = n_reals;                       // last realization with tile_base <= t
-        while (hi - lo > 1) {
-            const int mid = (lo + hi) >> 1;
-            if (tile_base[mid] <= t) lo = mid; else hi = mid;
-        }
-        const pyl_batch_real r = reals[lo];
+        const unsigned it = (unsigned)cur;
+        __syncthreads();
+        if (it >= total) break;
+        const BtPart pt = list[it];
+        const pyl_batch_real r = reals[pt.real];
+        const unsigned bin_end = min(offsets[pt.tile + 1], n_total);
+        const unsigned begin = min(offsets[pt.tile] + pt.first, bin_end);
+        const unsigned end = min(begin + pt.len, bin_end);
+        const BinShare sh{share + pt.shared * BT_SHARE_CELLS, done + pt.shared, pt.parts};
         const int nt = bt_nt(r.dims);
-        const int local = (int)(t - tile_base[lo]);
+        const int local = (int)(pt.tile - tile_base[pt.real]);
         const int o[3] = {(local / (nt * nt)) * TB, ((local / nt) % nt) * TB, (local % nt) * TB};
-        const bool inter = r.grid_interlaced != nullptr;
-        switch (r.mas * 2 + (inter ? 1 : 0)) {
-            case 2 * PYL_MAS_NGP:     bt_deposit_bin<PYL_MAS_NGP, false>(bsm, rec, begin, end, r, o); break;
-            case 2 * PYL_MAS_NGP + 1: bt_deposit_bin<PYL_MAS_NGP, true>(bsm, rec, begin, end, r, o); break;
-            case 2 * PYL_MAS_CIC:     bt_deposit_bin<PYL_MAS_CIC, false>(bsm, rec, begin, end, r, o); break;
-            case 2 * PYL_MAS_CIC + 1: bt_deposit_bin<PYL_MAS_CIC, true>(bsm, rec, begin, end, r, o); break;
-            case 2 * PYL_MAS_TSC:     bt_deposit_bin<PYL_MAS_TSC, false>(bsm, rec, begin, end, r, o); break;
-            case 2 * PYL_MAS_TSC + 1: bt_deposit_bin<PYL_MAS_TSC, true>(bsm, rec, begin, end, r, o); break;
-            case 2 * PYL_MAS_PCS:     bt_deposit_bin<PYL_MAS_PCS, false>(bsm, rec, begin, end, r, o); break;
-            default:                  bt_deposit_bin<PYL_MAS_PCS, true>(bsm, rec, begin, end, r, o); break;
+        const int pass = (int)pt.inter;
+        switch (r.mas * 2 + (r.grid_interlaced ? 1 : 0)) {
+            case 2 * PYL_MAS_NGP:     bt_deposit_bin<PYL_MAS_NGP, false>(bsm, rec, begin, end, r, o, 0, sh); break;
+            case 2 * PYL_MAS_NGP + 1: bt_deposit_bin<PYL_MAS_NGP, true>(bsm, rec, begin, end, r, o, pass, sh); break;
+            case 2 * PYL_MAS_CIC:     bt_deposit_bin<PYL_MAS_CIC, false>(bsm, rec, begin, end, r, o, 0, sh); break;
+            case 2 * PYL_MAS_CIC + 1: bt_deposit_bin<PYL_MAS_CIC, true>(bsm, rec, begin, end, r, o, pass, sh); break;
+            case 2 * PYL_MAS_TSC:     bt_deposit_bin<PYL_MAS_TSC, false>(bsm, rec, begin, end, r, o, 0, sh); break;
+            case 2 * PYL_MAS_TSC + 1: bt_deposit_bin<PYL_MAS_TSC, true>(bsm, rec, begin, end, r, o, pass, sh); break;
+            case 2 * PYL_MAS_PCS:     bt_deposit_bin<PYL_MAS_PCS, false>(bsm, rec, begin, end, r, o, 0, sh); break;
+            default:                  bt_deposit_bin<PYL_MAS_PCS, true>(bsm, rec, begin, end, r, o, pass, sh); break;
         }
     }
 }
 
 struct BtWs {
-    unsigned *counts, *offsets, *cursor, *counters;
+    unsigned *counts, *offsets, *cursor, *counters, *parts, *first_part, *done;
+    unsigned long long *adds, *share;
+    BtPart *list;
     float4 *rec;
-    size_t bytes;
+    size_t zero_bytes, bytes;
 };
 
 inline size_t bt_align(size_t v) { return (v + 255) / 256 * 256; }
@@ -498,7 +673,17 @@ BtWs bt_layout(void *base, unsigned total_tiles, long long total_particles)
     w.counts = (unsigned *)(b + o); o = bt_align(o + 4 * ((size_t)total_tiles + 1));
     w.offsets = (unsigned *)(b + o); o = bt_align(o + 4 * ((size_t)total_tiles + 1));
     w.cursor = (unsigned *)(b + o); o = bt_align(o + 4 * ((size_t)total_tiles + 1));
-    w.counters = (unsigned *)(b + o); o = bt_align(o + 4 * 4);
+    // counters, the count of additions and the parts' arrivals: zeroed together
+    const size_t shared = bt_max_shared(total_tiles, total_particles);
+    w.counters = (unsigned *)(b + o);
+    w.adds = (unsigned long long *)(b + o + 16);
+    w.done = (unsigned *)(b + o + 32);
+    w.zero_bytes = 32 + 4 * shared;
+    o = bt_align(o + w.zero_bytes);
+    w.share = (unsigned long long *)(b + o); o = bt_align(o + 8 * BT_SHARE_CELLS * shared);
+    w.parts = (unsigned *)(b + o); o = bt_align(o + 4 * ((size_t)total_tiles + 1));
+    w.first_part = (unsigned *)(b + o); o = bt_align(o + 4 * ((size_t)total_tiles + 1));
+    w.list = (BtPart *)(b + o); o = bt_align(o + sizeof(BtPart) * bt_max_parts(total_tiles));
     w.rec = (float4 *)(b + o); o = bt_align(o + 16 * (size_t)total_particles);
     w.bytes = o;
     return w;
@@ -567,7 +752,7 @@ extern "C" int pyl_ma_batch_tiled(const pyl_batch_real *reals, int n_reals, cons
     }
     cudaStream_t st = (cudaStream_t)stream;
     PYL_CUDA(cudaMemsetAsync(ws.counts, 0, 4 * ((size_t)total_tiles + 1), st));
-    PYL_CUDA(cudaMemsetAsync(ws.counters, 0, 16, st));
+    PYL_CUDA(cudaMemsetAsync(ws.counters, 0, ws.zero_bytes, st));
     if (n_items == 0) return PYL_OK;
     const unsigned grid = (unsigned)(num_sms() * ctas_per_sm);
     bt_count_kernel<<<grid, 1024, 0, st>>>(reals, items, n_items, tile_base, ws.counts, ws.counters);
@@ -578,9 +763,27 @@ extern "C" int pyl_ma_batch_tiled(const pyl_batch_real *reals, int n_reals, cons
     bt_place_kernel<<<grid, 1024, BT_PLACE_SMEM, st>>>(reals, items, n_items, tile_base, ws.cursor,
                                                        (unsigned)total_particles, ws.rec, ws.counters + 1);
     PYL_LAUNCH_CHECK();
+    const unsigned max_parts = (unsigned)bt_max_parts(total_tiles), sms = (unsigned)num_sms();
+    const size_t max_shared = bt_max_shared(total_tiles, total_particles);
+    const unsigned tb = (total_tiles + 255) / 256;
+    bt_adds_kernel<<<tb, 256, 0, st>>>(reals, n_reals, tile_base, total_tiles, ws.counts, ws.adds);
+    PYL_LAUNCH_CHECK();
+    bt_parts_kernel<<<tb, 256, 0, st>>>(reals, n_reals, tile_base, total_tiles, ws.counts, ws.adds, sms, ws.parts);
+    PYL_LAUNCH_CHECK();
+    bt_scan_kernel<<<1, 1024, 0, st>>>(ws.parts, total_tiles, ws.first_part, nullptr);
+    PYL_LAUNCH_CHECK();
+    bt_list_kernel<<<(total_tiles + 7) / 8, 256, 0, st>>>(
+        reals, n_reals, tile_base, total_tiles, ws.counts, ws.adds, sms, ws.first_part, max_parts,
+        (unsigned)max_shared, ws.counters + 3, ws.list);
+    PYL_LAUNCH_CHECK();
+    if (max_shared) {
+        bt_share_zero_kernel<<<dim3(8, (unsigned)max_shared), 256, 0, st>>>(ws.counters + 3, ws.share);
+        PYL_LAUNCH_CHECK();
+    }
     PYL_CUDA(ensure_smem(bt_deposit_kernel, BT_DEPOSIT_SMEM));
-    bt_deposit_kernel<<<(unsigned)num_sms(), 1024, BT_DEPOSIT_SMEM, st>>>(
-        reals, n_reals, tile_base, total_tiles, ws.offsets, (unsigned)total_particles, ws.rec, ws.counters + 2);
+    bt_deposit_kernel<<<sms, 1024, BT_DEPOSIT_SMEM, st>>>(
+        reals, tile_base, ws.list, ws.first_part + total_tiles, max_parts, ws.offsets, (unsigned)total_particles,
+        ws.rec, ws.share, ws.done, ws.counters + 2);
     PYL_LAUNCH_CHECK();
     return PYL_OK;
 }

@@ -177,6 +177,10 @@ __device__ __forceinline__ void fx_scatter_add(unsigned *acc, int base, const fl
         }
 }
 
+// Corner additions of the smallest part of a bin that is divided among CTAs: about 90 us
+// of them, where zeroing a bin's cells and adding them up takes about 10.
+constexpr long long PART_ADDS = 1 << 20;
+
 // COUNT: unweighted NGP adds one integer count per particle; otherwise every
 // corner adds its fixed-point weight (weighted NGP: C holds the scaled weight).
 // PRE: C[2] carries the factor 2^22 (see fx_corner).

@@ -174,7 +174,7 @@ extern "C" size_t pyl_ma_workspace_size(int64_t n_particles, int ndim, int dims,
         return sorted_workspace_bytes(n_particles, dims) + 256;
     if (s == PYL_STRATEGY_TILED && ndim == 3)
         return tiled_layout(nullptr, tiled_pass_len(n_particles), dims,
-                            owned_halo_floats(mas, dims, interlaced != 0)).bytes + 256;
+                            tiled_extra_bytes(tiled_pass_len(n_particles), mas, dims, interlaced != 0)).bytes + 256;
     return 256;
 }
 
@@ -214,7 +214,7 @@ extern "C" int pyl_ma(const float *pos, const float *weights, int64_t n, int ndi
                              nullptr, true, st);
     }
     if (s == PYL_STRATEGY_TILED && ndim != 3) s = PYL_STRATEGY_ATOMIC;
-    Owned ow{false, nullptr, 0, 0.0f, 0};
+    Owned ow{false, nullptr, 0, 0.0f, 0, false};
     const long long pass = tiled_pass_len(n);
     if (s == PYL_STRATEGY_TILED) {
         const size_t need = tiled_layout(nullptr, pass, dims).bytes;
@@ -222,10 +222,11 @@ extern "C" int pyl_ma(const float *pos, const float *weights, int64_t n, int ndi
             set_error("pyl_ma: tiled strategy needs " + std::to_string(need) + " workspace bytes");
             return PYL_ERR_WORKSPACE;
         }
-        // owned-cell write-out when the workspace also holds the halo blocks
-        const size_t need_owned =
-            tiled_layout(nullptr, pass, dims, owned_halo_floats(mas, dims, grid_interlaced != nullptr)).bytes;
-        ow.on = owned_applies(dims) && workspace_bytes >= need_owned;
+        // owned-cell write-out, or bins in parts, when the workspace also holds what they need
+        const size_t need_all =
+            tiled_layout(nullptr, pass, dims, tiled_extra_bytes(pass, mas, dims, grid_interlaced != nullptr)).bytes;
+        ow.on = owned_applies(dims) && workspace_bytes >= need_all;
+        ow.share = !owned_applies(dims) && workspace_bytes >= need_all;
     }
     int rc = PYL_OK;
     if (n > 0) {
@@ -337,7 +338,7 @@ int ma_overdensity_impl(const float *pos, const float *weights, int64_t n, float
     int s = pick_strategy(strategy, 3, dims, n);
     // the owned-cell write-out stores -1 + value into every cell: no fill pass
     // (with several tiled passes, the first stores and the others accumulate)
-    const Owned ow{s == PYL_STRATEGY_TILED && owned_applies(dims), nullptr, 1, -1.0f, 0};
+    const Owned ow{s == PYL_STRATEGY_TILED && owned_applies(dims), nullptr, 1, -1.0f, 0, !owned_applies(dims)};
     if (!ow.on) {
         const int blocks = grid_blocks(cells / 4 + 1, 256, 8);
         stage_mark(PYL_STAGE_FILL, true, st);

@@ -106,7 +106,8 @@ struct TiledWs {
     unsigned *hist, *total, *offsets;
     float4 *rec;                 // binned particles: x, y, z, weight
     float4 *tmp;                 // two-level placement: the coarse-block layout
-    float *halo;                 // owned-cell write-out: per-bin halo blocks
+    float *halo;                 // owned-cell write-out: per-bin halo blocks; else the grids'
+                                 // fixed-point words of bins in parts
     unsigned long long *same;    // coherence count of the histogram pass
     float *wsc;                  // weighted deposits: w_scale_kernel's 5 words
     int chunks;
@@ -116,7 +117,7 @@ struct TiledWs {
 
 inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
-inline TiledWs tiled_layout(void *base, long long n, int dims, size_t halo_floats = 0)
+inline TiledWs tiled_layout(void *base, long long n, int dims, size_t extra_bytes = 0)
 {
     TileGeom g = tile_geom(dims);
     TiledWs ws;
@@ -138,7 +139,7 @@ inline TiledWs tiled_layout(void *base, long long n, int dims, size_t halo_float
         off = align_up(off + sizeof(float4) * (size_t)n, 256);
     }
     ws.halo = (float *)(b + off);
-    off = align_up(off + sizeof(float) * halo_floats, 256);
+    off = align_up(off + extra_bytes, 256);
     ws.bytes = off;
     return ws;
 }
@@ -173,12 +174,52 @@ inline size_t owned_halo_floats(int mas, int dims, bool inter)
     return (size_t)(inter ? 2 : 1) * (size_t)tile_geom(dims).ntiles * (size_t)halo_cells(H);
 }
 
+// Parts of a bin's records.  Grids of fewer bins than half the SMs leave most of the chip
+// idle when a CTA takes a whole bin: its records then go to several CTAs, which add
+// their cells to 64-bit fixed-point words of the grid.  A part is an eighth of an SM's
+// share of all records, and at least PART_ADDS corner additions, with four times the
+// parts of an average bin for the heavier ones (the last part takes what is left).
+// Whole bins and parts measured: 512^3 particles on 64^3, PCS interlaced (8 bins, cells
+// past 512 that send whole bins to float32 sums): 1236 and 11.8 ms; 400^3 with masses on
+// 100^3, CIC (64 bins): 4.49 and 1.89; 256^3 on 128^3, CIC interlaced (64 bins): 0.58 and
+// 0.48.  With more bins the gain is a tenth or less (300^3 on 180^3, TSC, 216 bins: 0.94
+// and 0.84).
+struct BinParts {
+    unsigned len, parts;      // records of a part, CTAs per bin (1: whole bins)
+};
+
+inline BinParts bin_parts(long long n, int mas, int dims, bool inter)
+{
+    const long long nt = (dims + TB - 1) / TB, bins = nt * nt * nt, share = 8LL * num_sms();
+    const int S = mas == PYL_MAS_NGP ? 1 : mas;
+    const long long adds = (long long)S * S * S * (inter ? 2 : 1);
+    const long long len = std::max((n + share - 1) / share, PART_ADDS / adds);
+    if (2 * bins > num_sms() || n / bins < len) return BinParts{0u, 1u};
+    return BinParts{(unsigned)len, (unsigned)std::min(4 * (n / bins / len + 1), 65535LL)};
+}
+
+// Bytes of the fixed-point words of the grids (0: whole bins).
+inline size_t bin_share_bytes(long long n, int mas, int dims, bool inter)
+{
+    if (bin_parts(n, mas, dims, inter).parts == 1) return 0;
+    return sizeof(unsigned long long) * (size_t)dims * dims * dims * (inter ? 2 : 1);
+}
+
+// Bytes behind the records of a tiled workspace: the owned-cell halo blocks, or the words
+// of bins in parts.
+inline size_t tiled_extra_bytes(long long n, int mas, int dims, bool inter)
+{
+    return owned_applies(dims) ? sizeof(float) * owned_halo_floats(mas, dims, inter)
+                               : bin_share_bytes(n, mas, dims, inter);
+}
+
 struct Owned {
     bool on;             // false: atomic write-out of each bin with its halo
     float *halo;         // per-bin halo blocks (plain grid, then shifted grid)
     int fill_mode;       // 1: core = fill + value; 0: core = old + value
     float fill;
     long long stride;    // floats between the plain and the shifted grid's buffers
+    bool share;          // the workspace holds the words of bins in parts
 };
 
 // The whole tiled deposit of one MAS (histogram, scans, placement, per-bin deposit,
@@ -187,7 +228,7 @@ struct Owned {
 template <int MAS>
 int launch_tiled(const float *pos, const float *w, long long n, float *grid, float *grid2, int dims, float inv,
                  float halfcell, void *workspace, OutScale sc, cudaStream_t st, unsigned *err,
-                 const RsdArgs *rsd = nullptr, Owned ow = Owned{false, nullptr, 0, 0.0f, 0});
+                 const RsdArgs *rsd = nullptr, Owned ow = Owned{false, nullptr, 0, 0.0f, 0, false});
 
 extern template int launch_tiled<PYL_MAS_NGP>(const float *, const float *, long long, float *, float *, int, float, float, void *, OutScale,
                                   cudaStream_t, unsigned *, const RsdArgs *, Owned);

@@ -1154,6 +1154,40 @@ __device__ __forceinline__ float fx_value(unsigned w)
     return __fmul_rn(__uint2float_rn(w), FX_INV);
 }
 
+// Adds the bin's cells (with halo) into the grid: add(grid index, cell) for every cell;
+// threads walk the flattened cells 1024 apart with incremental (x, y, z) bin-local
+// indices.
+template <int MAS, bool INTER, typename Add>
+__device__ __forceinline__ void fx_each_cell(Add add, const int *o, int dims, bool interior)
+{
+    using FS = FxShape<MAS, INTER>;
+    constexpr int E = FS::E, CELLS = FS::CELLS;
+    constexpr int DZ = 1024 % E, DY = (1024 / E) % E, DX = 1024 / (E * E);
+    int lz = threadIdx.x % E, ly = (threadIdx.x / E) % E, lx = threadIdx.x / (E * E);
+    if (interior) {
+        const unsigned gbase = ((unsigned)o[0] * dims + o[1]) * dims + o[2];
+        for (int c = threadIdx.x; c < CELLS; c += 1024) {
+            add(gbase + ((unsigned)lx * dims + ly) * dims + lz, c);
+            lz += DZ;
+            ly += DY;
+            lx += DX;
+            if (lz >= E) { lz -= E; ly++; }
+            if (ly >= E) { ly -= E; lx++; }
+        }
+    } else {
+        const long long d = dims;
+        for (int c = threadIdx.x; c < CELLS; c += 1024) {
+            const long long gx = add_wrap(o[0], lx, d), gy = add_wrap(o[1], ly, d), gz = add_wrap(o[2], lz, d);
+            add((gx * d + gy) * d + gz, c);
+            lz += DZ;
+            ly += DY;
+            lx += DX;
+            if (lz >= E) { lz -= E; ly++; }
+            if (ly >= E) { ly -= E; lx++; }
+        }
+    }
+}
+
 // Adds the bin's cells (with halo) into the grid; threads walk the flattened
 // cells 1024 apart with incremental (x, y, z) bin-local indices.
 template <int MAS, bool INTER, bool FLOAT>
@@ -1190,6 +1224,44 @@ __device__ __forceinline__ void fx_write_out(const unsigned *smw, float *out, co
             if (lz >= E) { lz -= E; ly++; }
             if (ly >= E) { ly -= E; lx++; }
         }
+    }
+}
+
+// Write-out of a bin's part (BinParts): the cells' sums are added to the grid's 64-bit
+// fixed-point words, so the grid does not depend on how the records were divided or in
+// which order the parts end; share_finish_kernel adds the words to the grid.  A part
+// redone in float32 (a cell of 512 or more) goes there in the same units; float sums
+// of weights (any magnitude) and what is not finite go to the grid itself.
+template <int MAS, bool INTER, bool FLOAT>
+__device__ __forceinline__ void fx_share_out(const unsigned *smw, unsigned long long *share, float *out, const int *o,
+                                             int dims, bool interior, float scale, bool weighted)
+{
+    fx_each_cell<MAS, INTER>([&](long long i, int c) {
+        const unsigned w = smw[c];
+        if (w == 0u) return;
+        if (!FLOAT) {
+            atomicAdd(share + i, (unsigned long long)w);
+        } else {
+            const float v = __uint_as_float(w);
+            if (!weighted && fabsf(v) < 1e12f) atomicAdd(share + i, (unsigned long long)__float2ll_rn(__fmul_rn(v, FX_SCALE)));
+            else atomicAdd(out + i, __fmul_rn(v, scale));
+        }
+    }, o, dims, interior);
+}
+
+// grid += the words' values (NGP: counts, or fixed-point weights whose unit is in scale).
+template <int MAS>
+__global__ void __launch_bounds__(256) share_finish_kernel(const unsigned long long *__restrict__ share, long long n,
+                                                           OutScale sc, float *__restrict__ grid, const unsigned *err)
+{
+    if (*(const volatile unsigned *)err) return;        // the deposit left (some of) its bins out
+    const float scale = out_scale(sc);
+    const long long stride = (long long)gridDim.x * blockDim.x;
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
+        const long long w = (long long)share[i];
+        if (w == 0) continue;
+        const float v = __ll2float_rn(w);
+        grid[i] = __fadd_rn(grid[i], __fmul_rn(MAS == PYL_MAS_NGP ? v : __fmul_rn(v, FX_INV), scale));
     }
 }
 
@@ -1349,10 +1421,10 @@ __global__ void __launch_bounds__(256) halo_add_kernel(float *__restrict__ grid,
 
 // Both arithmetic modes of one grid: fixed point, float32 if that overflowed.
 // Returns false after a failed staging wait.
-template <int MAS, bool INTER, int R, int G, bool P2, bool TOT, bool FREE>
+template <int MAS, bool INTER, int R, int G, bool P2, bool TOT, bool FREE, bool PARTS>
 __device__ __forceinline__ bool fx_grid(const FxStage &sg, unsigned &q0, float inv, float halfcell, int dims,
                                         const int *o, unsigned *smw, float *out, bool interior, float scale,
-                                        const Owned &ow, float *halo_bin, const float *prev)
+                                        const Owned &ow, float *halo_bin, const float *prev, unsigned long long *share)
 {
     int st = 1;                                             // float32 from the start
     if (!(sg.use_float && *sg.use_float)) {
@@ -1362,6 +1434,7 @@ __device__ __forceinline__ bool fx_grid(const FxStage &sg, unsigned &q0, float i
     }
     if (st == 0) {
         if (ow.on) fx_store_owned<MAS, INTER, false>(smw, out, halo_bin, o, dims, scale, ow, prev, (float *)sg.inb);
+        else if (PARTS) fx_share_out<MAS, INTER, false>(smw, share, out, o, dims, interior, scale, sg.inv_w != nullptr);
         else fx_write_out<MAS, INTER, false>(smw, out, o, dims, interior, scale);
     } else {
         if (fx_accumulate<MAS, INTER, R, G, true, P2, false, FREE>(sg, q0, inv, halfcell, dims, o, smw) < 0) return false;
@@ -1370,17 +1443,22 @@ __device__ __forceinline__ bool fx_grid(const FxStage &sg, unsigned &q0, float i
         // float sums do not need
         const float fs = (MAS == PYL_MAS_NGP && sg.inv_w) ? __fmul_rn(scale, FX_SCALE) : scale;
         if (ow.on) fx_store_owned<MAS, INTER, true>(smw, out, halo_bin, o, dims, fs, ow, prev, (float *)sg.inb);
+        else if (PARTS) fx_share_out<MAS, INTER, true>(smw, share, out, o, dims, interior, fs, sg.inv_w != nullptr);
         else fx_write_out<MAS, INTER, true>(smw, out, o, dims, interior, fs);
     }
     __syncthreads();                                        // cells read before the next pass zeroes them
     return true;
 }
 
-template <int MAS, bool INTER, int R, bool P2, bool TOT, bool FREE>
+// PARTS: a CTA takes `part` records of a bin (BinParts), CTA blockIdx.y those from
+// blockIdx.y * part on and the last one all that are left, and adds its cells to the
+// words `share` of the grids (fx_share_out), the plain grid's first.  (A kernel of its
+// own: the 512^3 interlaced PCS deposit ran 3% slower with both in one.)
+template <int MAS, bool INTER, int R, bool P2, bool TOT, bool FREE, bool PARTS = false>
 __global__ void __launch_bounds__(1024) bin_deposit_fx_tma_kernel(
     const float4 *__restrict__ rec, const unsigned *__restrict__ offsets, TileGeom g, float inv,
     float halfcell, float *__restrict__ grid, float *__restrict__ grid2, OutScale sc, unsigned n_rec,
-    Owned ow, const float *inv_w, unsigned *err)
+    Owned ow, const float *inv_w, unsigned *err, unsigned part, unsigned long long *share)
 {
     // a bounded wait of the placement gave up (its records may be incomplete, and
     // stale records may lie outside the bin): deposit nothing, the error stands
@@ -1407,10 +1485,15 @@ __global__ void __launch_bounds__(1024) bin_deposit_fx_tma_kernel(
     bool have_prev = false;
     for (int k = 0; k < nbins; k++) {
         const long long tile = (long long)blockIdx.x * nbins + k;
-        const unsigned end = min(offsets[tile + 1], n_rec), begin = min(offsets[tile], end);
+        unsigned end = min(offsets[tile + 1], n_rec), begin = min(offsets[tile], end);
         int tx, ty, tz;
         tile_coords(tile, g, tx, ty, tz);
         if (tx >= g.nt || ty >= g.nt || tz >= g.nt) break;     // keys past the grid: no cells
+        if (PARTS) {
+            const unsigned long long b = begin + (unsigned long long)blockIdx.y * part;
+            begin = (unsigned)min(b, (unsigned long long)end);
+            if (blockIdx.y + 1 < gridDim.y) end = (unsigned)min(b + part, (unsigned long long)end);
+        }
         if (begin == end && !ow.on) return;                     // owned cells are stored even when empty
         const int o[3] = {tx * TB, ty * TB, tz * TB};
         const bool interior = o[0] + E <= dims && o[1] + E <= dims && o[2] + E <= dims &&
@@ -1426,11 +1509,13 @@ __global__ void __launch_bounds__(1024) bin_deposit_fx_tma_kernel(
         sg.err = err;
         float *hb = ow.on && HC > 0 ? ow.halo + tile * HC : nullptr;
         const float *prev = have_prev && hb ? hb - HC : nullptr;
-        if (!fx_grid<MAS, INTER, R, 0, P2, TOT, FREE>(sg, q0, inv, halfcell, dims, o, smw, grid, interior, scale, ow, hb, prev))
+        if (!fx_grid<MAS, INTER, R, 0, P2, TOT, FREE, PARTS>(sg, q0, inv, halfcell, dims, o, smw, grid, interior, scale, ow, hb,
+                                                             prev, share))
             return;
         if (INTER &&
-            !fx_grid<MAS, INTER, R, 1, P2, TOT, FREE>(sg, q0, inv, halfcell, dims, o, smw, grid2, interior, scale, ow,
-                                       hb ? hb + ow.stride : nullptr, prev ? prev + ow.stride : nullptr))
+            !fx_grid<MAS, INTER, R, 1, P2, TOT, FREE, PARTS>(sg, q0, inv, halfcell, dims, o, smw, grid2, interior, scale, ow,
+                                       hb ? hb + ow.stride : nullptr, prev ? prev + ow.stride : nullptr,
+                                       PARTS ? share + (size_t)dims * dims * dims : nullptr))
             return;
         have_prev = true;
     }
@@ -1467,11 +1552,31 @@ int launch_deposit_fx(const TiledWs &ws, TileGeom g, float inv, float halfcell, 
                                        : bin_deposit_fx_tma_kernel<MAS, I, RR, true, false, false>)
                                 : (tot ? bin_deposit_fx_tma_kernel<MAS, I, RR, false, true, false>
                                        : bin_deposit_fx_tma_kernel<MAS, I, RR, false, false, false>));
+        const unsigned ctas = (unsigned)(ow.on ? g.ntiles / OWN_Z : g.ntiles);
+        BinParts bp{0u, 1u};
+        unsigned long long *share = nullptr;
+        if (ow.share) {
+            bp = bin_parts(ws.n, MAS, g.dims, I);
+            const size_t bytes = bin_share_bytes(ws.n, MAS, g.dims, I);
+            if (bytes) {
+                share = (unsigned long long *)ws.halo;
+                kern = bin_deposit_fx_tma_kernel<MAS, I, RR, false, false, false, true>;
+                PYL_CUDA(cudaMemsetAsync(share, 0, bytes, st));
+            }
+        }
         const size_t smem = FS::SMEM + 2 * (size_t)R * 16;
         PYL_CUDA(ensure_smem(kern, smem));
-        const unsigned ctas = (unsigned)(ow.on ? g.ntiles / OWN_Z : g.ntiles);
-        kern<<<ctas, 1024, smem, st>>>(ws.rec, ws.offsets, g, inv, halfcell, grid, grid2, sc, ws.n, ow, inv_w, err);
+        kern<<<dim3(ctas, bp.parts), 1024, smem, st>>>(ws.rec, ws.offsets, g, inv, halfcell, grid, grid2, sc, ws.n, ow,
+                                                       inv_w, err, bp.len, share);
         PYL_LAUNCH_CHECK();
+        if (share) {
+            const long long cells = (long long)g.dims * g.dims * g.dims;
+            for (int k = 0; k < (I ? 2 : 1); k++) {
+                share_finish_kernel<MAS><<<grid_blocks(cells, 256), 256, 0, st>>>(share + k * cells, cells, sc,
+                                                                                  k ? grid2 : grid, err);
+                PYL_LAUNCH_CHECK();
+            }
+        }
         if constexpr (FS::H > 0) {
             if (ow.on) {
                 stage_mark(PYL_STAGE_DEPOSIT, false, st);
