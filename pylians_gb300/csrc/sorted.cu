@@ -9,24 +9,20 @@
 //      ranks each tile's keys stably (warp match + per-warp digit counts) and
 //      stages them in shared memory so global writes are coalesced.  Equal keys
 //      keep increasing particle index.
-//   3. run table: for every cell the [start, end) range of its particles in the
-//      sorted order (empty cells keep the all-ones marker).
-//   4. the particles' positions (and weights) gathered into sorted order.
-//   5. gather deposit: one thread per output cell walks the S^3 neighbouring
-//      base cells in a fixed order and, within each run, the particles in index
-//      order, adding the weight of its corner; the CTA stages the particles of
-//      its base cells in shared memory with their weights computed once per x
-//      offset (sd_deposit_kernel).  The interlaced grid runs
-//      steps 1-5 again on the shifted positions (its own sort), so its cells
-//      also visit S^3 base cells (a gather over the plain grid's sort visited
-//      (S+1)^3 and checked each corner: 4x the work for TSC).
-//      No atomics: every cell's sum has one fixed order, so the grid is
-//      bit-reproducible whatever the launch configuration; NGP sums each cell's
-//      particles in index order, exactly the serial reference loop.
+//   3. the particles' positions (and weights) gathered into sorted order, and a table of
+//      where each column (ix, iy) and every SD_Z cells along it start there.
+//   4. deposit (sd_deposit_kernel): a thread walks a base column (ix, iy) along z and
+//      keeps the S^3 sums that its particles add to, S output layers of S x S columns,
+//      in registers; at every z the layer that no later particle reaches is exchanged
+//      through shared memory and each output cell adds its S^2 base columns' values.
+//      The interlaced grid runs steps 1-4 again on the shifted positions (its own sort).
+//      No atomics: every cell's sum has one fixed order (base columns by (l, m), within
+//      a column particles by z and index), so the grid is bit-reproducible whatever the
+//      launch configuration; NGP adds each cell's particles in index order onto the
+//      grid's value, exactly the serial reference loop.
 // Limits: dims^3 <= 2^32 (dims <= 1625) and fewer than 2^32 particles.
 #include <cuda_runtime.h>
 
-#include <atomic>
 #include <string>
 
 #include "common.cuh"
@@ -43,7 +39,6 @@ constexpr int RS_WARPS = RS_THREADS / 32;
 constexpr int SCAN_THREADS = 1024;
 constexpr int SCAN_ITEMS = 4;
 constexpr int SCAN_BLOCK = SCAN_THREADS * SCAN_ITEMS;  // 4096 entries per scan block
-constexpr unsigned EMPTY = 0xffffffffu;
 
 template <int MAS>
 __device__ __forceinline__ int sd_first(float p, float inv)
@@ -60,50 +55,6 @@ __device__ __forceinline__ int sd_first(float p, float inv)
     }
     if (MAS == PYL_MAS_TSC) return fi - 1 + (frac >= 0.5f ? 1 : 0);
     return fi - 1;
-}
-
-// Weight of support cell j (0 <= j < S) of one coordinate and the first cell;
-// the same float arithmetic as the scatter kernels (mas.cu axis_weights).
-template <int MAS>
-__device__ __forceinline__ float sd_weight(float p, float inv, int j, int *first)
-{
-    const float dist = __fmul_rn(p, inv);
-    if (MAS == PYL_MAS_NGP) {
-        *first = sd_first<MAS>(p, inv);
-        return 1.0f;
-    } else if (MAS == PYL_MAS_CIC) {
-        const float t = truncf(dist);
-        const float u = __fsub_rn(dist, t);
-        *first = __float2int_rz(t);
-        return j == 0 ? __fsub_rn(1.0f, u) : u;
-    } else if (MAS == PYL_MAS_TSC) {
-        const float fl = floorf(dist);
-        const float frac = __fsub_rn(dist, fl);
-        *first = __float2int_rz(fl) - 1 + (frac >= 0.5f ? 1 : 0);
-        const float fmn = __fsub_rn(__fadd_rn(fl, frac >= 0.5f ? 1.0f : 0.0f), 2.0f);
-        const float diff = fabsf(__fsub_rn(__fadd_rn(fmn, (float)(j + 1)), dist));
-        if (diff < 0.5f) return __fsub_rn(0.75f, __fmul_rn(diff, diff));
-        if (diff < 1.5f) {
-            const float t = __fsub_rn(1.5f, diff);
-            return __fmul_rn(__fmul_rn(0.5f, t), t);
-        }
-        return 0.0f;
-    } else {
-        const float fl = floorf(dist);
-        *first = __float2int_rz(fl) - 1;
-        const float fmn = __fsub_rn(fl, 2.0f);
-        const float d = fabsf(__fsub_rn(__fadd_rn(fmn, (float)(j + 1)), dist));
-        if (d < 1.0f) {
-            const float a = __fmul_rn(__fmul_rn(6.0f, d), d);
-            const float b = __fmul_rn(__fmul_rn(__fmul_rn(3.0f, d), d), d);
-            return __fdiv_rn(__fadd_rn(__fsub_rn(4.0f, a), b), 6.0f);
-        }
-        if (d < 2.0f) {
-            const float t = __fsub_rn(2.0f, d);
-            return __fdiv_rn(__fmul_rn(__fmul_rn(t, t), t), 6.0f);
-        }
-        return 0.0f;
-    }
 }
 
 // ---- 1. keys --------------------------------------------------------------
@@ -310,26 +261,24 @@ __global__ void __launch_bounds__(RS_THREADS) rs_scatter_kernel(
     }
 }
 
-// ---- 3. run table -------------------------------------------------------------
-__global__ void __launch_bounds__(256) sd_runs_kernel(const unsigned *__restrict__ keys, long long n,
-                                                      uint2 *__restrict__ runs)
+// ---- 3. column starts ----------------------------------------------------------
+constexpr int SD_Z = 8;           // cells along z of a segment
+
+// start[t] = first sorted particle with key >= (t / nseg) * dims + (t % nseg) * SD_Z, for
+// t = 0 .. dims^2 * nseg (the last entry: n).
+__global__ void __launch_bounds__(256) sd_start_kernel(const unsigned *__restrict__ keys, long long n, unsigned dims,
+                                                       unsigned nseg, long long entries, unsigned *__restrict__ start)
 {
     const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x; j < n; j += stride) {
-        const unsigned k = keys[j];
-        if (j == 0 || keys[j - 1] != k) runs[k].x = (unsigned)j;
-        if (j == n - 1 || keys[j + 1] != k) runs[k].y = (unsigned)(j + 1);
+    for (long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x; j <= n; j += stride) {
+        // entries after the previous particle's segment, up to this one's
+        long long t = j == 0 ? 0 : (long long)(keys[j - 1] / dims) * nseg + keys[j - 1] % dims / SD_Z + 1;
+        const long long e = j == n ? entries : (long long)(keys[j] / dims) * nseg + keys[j] % dims / SD_Z;
+        for (; t <= e; t++) start[t] = (unsigned)j;
     }
 }
 
-__global__ void __launch_bounds__(256) sd_fill2_kernel(uint2 *__restrict__ p, long long n)
-{
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride)
-        p[i] = make_uint2(EMPTY, EMPTY);
-}
-
-// ---- 4. positions in sorted order -------------------------------------------
+// ---- 3. positions in sorted order -------------------------------------------
 template <bool SHIFT>
 __global__ void __launch_bounds__(256) sd_gather_kernel(const float *__restrict__ pos, const float *__restrict__ w,
                                                         const unsigned *__restrict__ vals, long long n,
@@ -349,191 +298,176 @@ __global__ void __launch_bounds__(256) sd_gather_kernel(const float *__restrict_
     }
 }
 
-// ---- 5. gather deposit ----------------------------------------------------------
-// Cell (x, y, z) sums, over base cells c - (l, m, q) with offsets 0..S-1 per axis
-// in that order and each run's particles in index order, the weight of its corner
-// ((c0 c1) c2, times the weight), in float32 adds: a fixed order, so the grid is
-// the same bits on every run.  The half-cell-shifted grid runs the same gather on
-// its own sort of the shifted positions (sorted_pass<MAS, true>).
-// scale/base: out = (fold ? out : 0) + sum in fixed order, then
-//   (fold ? sum : out_old + sum * scale).
+// ---- 4. deposit --------------------------------------------------------------------
+// A CTA of 16 x 32 threads takes the base columns (X0 - (S-1) + tx, Y0 - (S-1) + ty) and
+// `zs` output layers; its output cells are those whose S x S base columns are all its
+// own.  Thread (tx, ty) walks its column's particles from base layer z0 - (S-1) on: at
+// base layer z they add to the output layers z .. z + S-1 of the S x S columns from it,
+// acc[l][m][q] (q turns with z: the loop is unrolled by S).  After layer z its S^2 sums
+// are complete and go to shared memory; every few layers (ZB) the CTA meets, and output cell
+// (tx, ty) adds those of the columns (tx - l, ty - m).  Outputs are written 8 layers at a
+// time, whole sectors.  Two particles ahead are in flight.
+// Bound by instructions of half-empty warps (at one particle per cell the fullest of a
+// warp's 32 cells holds 3.9: 13 lanes in use, 60 % of issue slots, 30 warps per SM):
+// 256^3 TSC of 256^3 particles 0.81 ms; 1.89 ms for a gather that visited S^3 base cells
+// for each output cell.  More base layers between meetings leave one CTA per SM (1.26 ms).
+constexpr int SDX = 16, SDY = 32;
+constexpr int SD_CTA_LAYERS = 32;
 
-// One (l, m) of one cell straight from the runs and the sorted positions.
-template <int MAS, bool WEIGHTED>
-__device__ __forceinline__ float sd_direct_lm(const float4 *__restrict__ spos, const uint2 *__restrict__ runs,
-                                              long long row, int z, int dims, float inv, int l, int m, float acc)
-{
-    constexpr int S = MAS == PYL_MAS_NGP ? 1 : MAS;
-#pragma unroll
-    for (int q = 0; q < S; q++) {
-        const uint2 rr = runs[row + wrap_index(z - q, dims)];
-        if (rr.x == EMPTY) continue;
-        for (unsigned j = rr.x; j < rr.y; j++) {
-            const float4 p = spos[j];
-            int f;
-            const float c0 = sd_weight<MAS>(p.x, inv, l, &f);
-            const float c1 = sd_weight<MAS>(p.y, inv, m, &f);
-            const float c2 = sd_weight<MAS>(p.z, inv, q, &f);
-            float v = MAS == PYL_MAS_NGP ? 1.0f : __fmul_rn(__fmul_rn(c0, c1), c2);
-            if (WEIGHTED) v = MAS == PYL_MAS_NGP ? p.w : __fmul_rn(v, p.w);
-            acc = __fadd_rn(acc, v);
-        }
-    }
-    return acc;
-}
-
-constexpr int SDT_CAP = 1024;      // particles a CTA stages per x offset l (shared-memory capacity)
-std::atomic<int> g_sd_stage_cap{SDT_CAP};   // pyl_sorted_set_stage_limit
-
-// Of one staged particle: the products (x weight at offset l) (y weight at offset
-// m) for m = 0..S-1, the z weights at offsets 0..S-1 (and the weight).
-template <int MAS, bool WEIGHTED>
-struct SdStage {
-    static constexpr int S = MAS == PYL_MAS_NGP ? 1 : MAS;
-    static constexpr int NV = 2 * S + (WEIGHTED ? 1 : 0);
-    static constexpr int RY = 8 + S - 1, W = 32 + S - 1;   // base rows along y, base cells along z
-    static constexpr int NC = RY * W;                       // window cells of one l
+template <int MAS>
+struct SdShape {
+    static constexpr int S = MAS, NT = SDX * SDY, FL = 8, PAD = 4;
+    static constexpr int ZB = S == 2 ? 8 : S;               // base layers between two meetings (S divides it)
+    static constexpr size_t SMEM = sizeof(float) * (ZB * S * S * NT + FL * (NT + PAD));
 };
 
-// A CTA takes the 32 x 8 cells (z, y) of one x plane; block (32, 8), grid
-// (ceil(dims / 32), ceil(dims / 8), dims).  For each x offset l the CTA reads the
-// runs of the (8 + S - 1) x (32 + S - 1) base cells its cells reach in plane
-// x - l, places their particles in shared memory by a block scan, and computes
-// each staged particle's S (x, y) weight products and S z weights once (all S
-// weights of an axis from one axis_weights, the arithmetic of sd_weight),
-// instead of once for each of the S^2 cells of the plane that it reaches.
-// Every cell then sums its base cells' staged particles in the order above, with
-// the same products and adds as sd_direct_lm, which takes over for an l whose
-// window holds more than cap (at most SDT_CAP) particles.
 template <int MAS, bool WEIGHTED>
-__global__ void __launch_bounds__(256) sd_deposit_kernel(const float4 *__restrict__ spos,
-                                                         const uint2 *__restrict__ runs, int dims, float inv,
-                                                         float *__restrict__ out, float scale_h,
-                                                         const float *__restrict__ scale_d, int fold,
-                                                         unsigned cap)
+__global__ void __launch_bounds__(SDX * SDY, MAS == PYL_MAS_PCS ? 1 : 2) sd_deposit_kernel(
+    const float4 *__restrict__ spos, const unsigned *__restrict__ keys, const unsigned *__restrict__ start, int dims,
+    int nseg, int zs, float inv, float *__restrict__ out, float scale_h, const float *__restrict__ scale_d, int fold)
 {
-    using ST = SdStage<MAS, WEIGHTED>;
-    constexpr int S = ST::S, NV = ST::NV, W = ST::W, NC = ST::NC;
-    constexpr int CPT = (NC + 255) / 256;                   // window cells a thread reads
-    __shared__ unsigned s_off[NC + 1];                      // staged start of each window cell
-    __shared__ unsigned s_rx[NC];                           // its first particle in sorted order
-    __shared__ float s_e[SDT_CAP * NV];
-    __shared__ unsigned s_wsum[8];
-    const int tid = threadIdx.y * 32 + threadIdx.x, lane = threadIdx.x, warp = threadIdx.y;
-    const int z0 = blockIdx.x * 32, y0 = blockIdx.y * 8;
-    const int z = z0 + threadIdx.x, y = y0 + threadIdx.y, x = blockIdx.z;
-    const bool live = z < dims && y < dims;
-    const long long d = dims;
-    const long long cell = ((long long)x * d + y) * d + z;
-    float acc = (fold && live) ? out[cell] : 0.0f;
-#pragma unroll 1
-    for (int l = 0; l < S; l++) {
-        const long long plane = (long long)wrap_index(x - l, dims) * d;
-        // 1. runs of this thread's window cells tid * CPT + k (row r = c / W, cell
-        //    i = c % W: base cell (y0 - (S - 1) + r, z0 - (S - 1) + i)); cells past
-        //    the grid's end serve no live cell and stay empty
-        unsigned cnt[CPT], sum = 0;
+    using SH = SdShape<MAS>;
+    constexpr int S = SH::S, NT = SH::NT, H = S - 1, FL = SH::FL, PAD = SH::PAD, ZB = SH::ZB;
+    extern __shared__ float sd_sm[];
+    float *ex = sd_sm;                                       // [ZB][S * S][NT]
+    float *res = sd_sm + ZB * S * S * NT;                    // [FL][NT + PAD]
+    const int ty = threadIdx.x, tx = threadIdx.y, tid = tx * SDY + ty;
+    const int X0 = blockIdx.z * (SDX - H), Y0 = blockIdx.y * (SDY - H);
+    const int z0 = blockIdx.x * zs, z1 = min(dims, z0 + zs);
+    const int bx = wrap_index(X0 - H + tx, dims), by = wrap_index(Y0 - H + ty, dims);
+    const unsigned col = (unsigned)bx * (unsigned)dims + (unsigned)by;
+    const float scale = scale_d ? *scale_d : scale_h;
+    // first sorted particle of this column at or past layer z
+    auto first_from = [&](int z) {
+        const unsigned *t = start + (long long)col * nseg + z / SD_Z;
+        unsigned lo = t[0], hi = t[1];
+        const unsigned key = col * (unsigned)dims + (unsigned)z;
+        while (lo < hi) {
+            const unsigned mid = lo + (hi - lo) / 2;
+            if (keys[mid] < key) lo = mid + 1; else hi = mid;
+        }
+        return lo;
+    };
+    const unsigned col_end = start[(long long)(col + 1) * nseg];
+    const int X = X0 + tx - H, Y = Y0 + ty - H;             // output column (tx, ty >= H)
+    const bool live = tx >= H && ty >= H && X < dims && Y < dims;
+    float acc[S][S][S];
 #pragma unroll
-        for (int k = 0; k < CPT; k++) {
-            const int c = tid * CPT + k;
-            cnt[k] = 0;
-            if (c < NC) {
-                const int yb = y0 - (S - 1) + c / W, zb = z0 - (S - 1) + c % W;
-                unsigned rx = 0;
-                if (yb < dims && zb < dims) {
-                    const uint2 rr = runs[(plane + wrap_index(yb, dims)) * d + wrap_index(zb, dims)];
-                    if (rr.x != EMPTY) { cnt[k] = rr.y - rr.x; rx = rr.x; }
+    for (int l = 0; l < S; l++)
+#pragma unroll
+        for (int m = 0; m < S; m++)
+#pragma unroll
+            for (int q = 0; q < S; q++) acc[l][m][q] = 0.0f;
+
+    // particles j, j + 1 of the column; layer: base layer of the first (-1: none left)
+    unsigned j = 0;
+    float4 p = make_float4(0.0f, 0.0f, 0.0f, 0.0f), p2 = p;
+    int layer = -1;
+    auto layer_of = [&]() { return j < col_end ? wrap_index(sd_first<MAS>(p.z, inv), dims) : -1; };
+    const int layers = z1 - z0 + H;
+    for (int k0 = 0; k0 < layers; k0 += ZB) {                // base layers z0 - H + k0 ..
+#pragma unroll 1
+        for (int g = 0; g < ZB; g += S) {
+#pragma unroll
+            for (int u = 0; u < S; u++) {
+                const int k = k0 + g + u;
+                if (k >= layers) break;
+                const int zb = wrap_index(z0 - H + k, dims);
+                if (k == 0 || zb == 0) {
+                    j = first_from(zb);
+                    if (j < col_end) p = __ldg(spos + j);
+                    if (j + 1 < col_end) p2 = __ldg(spos + j + 1);
+                    layer = layer_of();
                 }
-                s_rx[c] = rx;
-            }
-            sum += cnt[k];
-        }
-        // 2. block exclusive scan of the thread sums
-        unsigned inc = sum;
+                while (layer == zb) {
+                    const float4 r = p;
+                    p = p2;
+                    j++;
+                    if (j + 1 < col_end) p2 = __ldg(spos + j + 1);
+                    layer = layer_of();
+                    float cx[S], cy[S], cz[S];
+                    axis_weights<MAS>(r.x, inv, cx);
+                    axis_weights<MAS>(r.y, inv, cy);
+                    axis_weights<MAS>(r.z, inv, cz);
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const unsigned t = __shfl_up_sync(0xffffffffu, inc, o);
-            if (lane >= o) inc += t;
-        }
-        if (lane == 31) s_wsum[warp] = inc;
-        __syncthreads();
-        unsigned before = 0, total = 0;
+                    for (int l = 0; l < S; l++)
 #pragma unroll
-        for (int w2 = 0; w2 < 8; w2++) {
-            const unsigned v = s_wsum[w2];
-            before += w2 < warp ? v : 0u;
-            total += v;
-        }
-        unsigned run = before + inc - sum;
+                        for (int m = 0; m < S; m++) {
+                            float c = __fmul_rn(cx[l], cy[m]);
+                            if (WEIGHTED) c = __fmul_rn(c, r.w);
 #pragma unroll
-        for (int k = 0; k < CPT; k++) {
-            const int c = tid * CPT + k;
-            if (c < NC) s_off[c] = run;
-            run += cnt[k];
-        }
-        if (tid == 0) s_off[NC] = total;
-        __syncthreads();                                    // s_wsum reads done, s_off / s_rx written
-        if (total > cap) {                                  // the same for the whole CTA (cap <= SDT_CAP)
-            if (live)
-#pragma unroll 1
-                for (int m = 0; m < S; m++)
-                    acc = sd_direct_lm<MAS, WEIGHTED>(spos, runs, (plane + wrap_index(y - m, dims)) * d, z, dims,
-                                                      inv, l, m, acc);
-            __syncthreads();
-            continue;
-        }
-        // 3. stage: particle t of the window is particle t - s_off[c] of window cell c
-        for (unsigned t = tid; t < total; t += 256) {
-            int lo = 0, hi = NC;                            // s_off[lo] <= t < s_off[hi]
-            while (hi - lo > 1) {
-                const int mid = (lo + hi) >> 1;
-                if (s_off[mid] <= t) lo = mid; else hi = mid;
-            }
-            const float4 p = spos[s_rx[lo] + (t - s_off[lo])];
-            float *e = s_e + t * NV;
-            if (MAS == PYL_MAS_NGP) {
-                e[0] = e[1] = 1.0f;
-            } else {
-                float cx[S], cy[S], cz[S];
-                axis_weights<MAS>(p.x, inv, cx);
-                axis_weights<MAS>(p.y, inv, cy);
-                axis_weights<MAS>(p.z, inv, cz);
-                float c0 = cx[0];
+                            for (int q = 0; q < S; q++) acc[l][m][(u + q) % S] = __fmaf_rn(c, cz[q], acc[l][m][(u + q) % S]);
+                        }
+                }
+                // the layer is complete: its sums out, its place free for layer k + S
+                float *e = ex + (g + u) * S * S * NT + tid;
 #pragma unroll
-                for (int j = 1; j < S; j++) c0 = l == j ? cx[j] : c0;
+                for (int l = 0; l < S; l++)
 #pragma unroll
-                for (int m = 0; m < S; m++) e[m] = __fmul_rn(c0, cy[m]);
-#pragma unroll
-                for (int q = 0; q < S; q++) e[S + q] = cz[q];
-            }
-            if (WEIGHTED) e[2 * S] = p.w;
-        }
-        __syncthreads();
-        // 4. each cell: base rows y - m, base cells z - q, particles in index order
-        if (live) {
-#pragma unroll 1
-            for (int m = 0; m < S; m++) {
-#pragma unroll
-                for (int q = 0; q < S; q++) {
-                    const int c = (warp + (S - 1) - m) * W + lane + (S - 1) - q;
-                    const unsigned a = s_off[c], b = s_off[c + 1];
-                    for (unsigned t = a; t < b; t++) {
-                        const float *e = s_e + t * NV;
-                        float v = MAS == PYL_MAS_NGP ? 1.0f : __fmul_rn(e[m], e[S + q]);
-                        if (WEIGHTED) v = MAS == PYL_MAS_NGP ? e[2 * S] : __fmul_rn(v, e[2 * S]);
-                        acc = __fadd_rn(acc, v);
+                    for (int m = 0; m < S; m++) {
+                        e[(l * S + m) * NT] = acc[l][m][u];
+                        acc[l][m][u] = 0.0f;
                     }
-                }
             }
         }
-        __syncthreads();                                    // before the next l restages
+        __syncthreads();
+        // output layers z0 + k - H of the base layers k since the last meeting; eight of
+        // them, or the last ones, are written together
+        for (int u = 0; u < ZB; u++) {
+            const int zi = k0 + u - H;
+            if (zi < 0 || k0 + u >= layers) continue;
+            if (live) {
+                float v = 0.0f;
+                const float *f = ex + u * S * S * NT + tid;
+#pragma unroll
+                for (int l = 0; l < S; l++)
+#pragma unroll
+                    for (int m = 0; m < S; m++) v = __fadd_rn(v, f[(l * S + m) * NT - l * SDY - m]);
+                res[(zi % FL) * (NT + PAD) + tid] = v;
+            }
+            if (zi % FL == FL - 1 || z0 + zi + 1 == z1) {    // uniform
+                __syncthreads();
+                const int zf = zi - zi % FL;
+                for (int i = tid; i < NT * FL; i += NT) {
+                    const int row = i / FL, dz = i % FL, rx = row / SDY, ry = row % SDY;
+                    const int ox = X0 + rx - H, oy = Y0 + ry - H;
+                    if (rx < H || ry < H || ox >= dims || oy >= dims || zf + dz > zi) continue;
+                    const float v = res[dz * (NT + PAD) + row];
+                    float *c = out + ((long long)ox * dims + oy) * dims + z0 + zf + dz;
+                    if (fold) *c = __fadd_rn(*c, v);
+                    else if (v != 0.0f) *c = __fadd_rn(*c, __fmul_rn(v, scale));
+                }
+                __syncthreads();
+            }
+        }
+        __syncthreads();                                     // ex is read
     }
-    if (!live) return;
-    if (fold) {
-        out[cell] = acc;
-    } else if (acc != 0.0f) {
-        const float s = scale_d ? *scale_d : scale_h;
-        out[cell] = __fadd_rn(out[cell], __fmul_rn(acc, s));
+}
+
+// NGP: a thread per cell finds its particles in the column's segment (cell = key) and
+// adds them in index order onto the grid's value (fold), as the serial loop does.
+template <bool WEIGHTED>
+__global__ void __launch_bounds__(256) sd_ngp_kernel(const float4 *__restrict__ spos, const unsigned *__restrict__ keys,
+                                                     const unsigned *__restrict__ start, int dims, int nseg,
+                                                     long long cells, float *__restrict__ out, float scale_h,
+                                                     const float *__restrict__ scale_d, int fold)
+{
+    const long long stride = (long long)gridDim.x * blockDim.x;
+    const float scale = scale_d ? *scale_d : scale_h;
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < cells; i += stride) {
+        const unsigned key = (unsigned)i;
+        const unsigned *t = start + (long long)(key / (unsigned)dims) * nseg + key % (unsigned)dims / SD_Z;
+        unsigned lo = t[0], hi = t[1];
+        const unsigned end = hi;
+        while (lo < hi) {
+            const unsigned mid = lo + (hi - lo) / 2;
+            if (keys[mid] < key) lo = mid + 1; else hi = mid;
+        }
+        if (lo >= end || keys[lo] != key) continue;
+        float v = fold ? out[i] : 0.0f;
+        for (; lo < end && keys[lo] == key; lo++) v = __fadd_rn(v, WEIGHTED ? __ldg(spos + lo).w : 1.0f);
+        if (fold) out[i] = v;
+        else if (v != 0.0f) out[i] = __fadd_rn(out[i], __fmul_rn(v, scale));
     }
 }
 
@@ -541,17 +475,17 @@ inline size_t al(size_t v) { return (v + 255) / 256 * 256; }
 
 struct SortedWs {
     unsigned *k0, *v0, *k1, *v1, *hist, *partial;
-    uint2 *runs;
+    unsigned *start;
     float4 *spos;
     unsigned tiles;
-    long long hist_len, parts;
+    long long hist_len, parts, entries;      // entries: dims^2 * segments of a column
     size_t bytes;
 };
 
 SortedWs sorted_layout(void *base, long long n, int dims)
 {
     SortedWs w;
-    const long long cells = (long long)dims * dims * dims;
+    w.entries = (long long)dims * dims * ((dims + SD_Z - 1) / SD_Z);
     w.tiles = (unsigned)((n + RS_TILE - 1) / RS_TILE);
     w.hist_len = 256LL * w.tiles;
     w.parts = (w.hist_len + SCAN_BLOCK - 1) / SCAN_BLOCK;
@@ -563,7 +497,7 @@ SortedWs sorted_layout(void *base, long long n, int dims)
     w.v1 = (unsigned *)(b + o); o = al(o + 4 * (size_t)n);
     w.hist = (unsigned *)(b + o); o = al(o + 4 * (size_t)w.hist_len);
     w.partial = (unsigned *)(b + o); o = al(o + 4 * (size_t)w.parts);
-    w.runs = (uint2 *)(b + o); o = al(o + 8 * (size_t)cells);
+    w.start = (unsigned *)(b + o); o = al(o + 4 * (size_t)(w.entries + 1));
     w.spos = (float4 *)(b + o); o = al(o + 16 * (size_t)n);
     w.bytes = o;
     return w;
@@ -576,8 +510,8 @@ inline unsigned blocks_for(long long n, int threads, int per_sm)
     return (unsigned)(b < 1 ? 1 : (b > cap ? cap : b));
 }
 
-// One grid: keys of the (shifted, for SHIFT) positions, stable radix sort, runs,
-// positions gathered into sorted order, gather deposit.
+// One grid: keys of the (shifted, for SHIFT) positions, stable radix sort, column starts,
+// positions gathered into sorted order, deposit.
 template <int MAS, bool SHIFT>
 int sorted_pass(const float *pos, const float *w, long long n, float *out, int dims, float inv, float halfcell,
                 const SortedWs &ws, float scale_h, const float *scale_d, bool fold, cudaStream_t st)
@@ -603,19 +537,31 @@ int sorted_pass(const float *pos, const float *w, long long n, float *out, int d
         unsigned *t = kin; kin = kout; kout = t;
         t = vin; vin = vout; vout = t;
     }
-    sd_fill2_kernel<<<blocks_for(cells, 256, 16), 256, 0, st>>>(ws.runs, cells);
-    PYL_LAUNCH_CHECK();
-    sd_runs_kernel<<<blocks_for(n, 256, 16), 256, 0, st>>>(kin, n, ws.runs);
+    const int nseg = (dims + SD_Z - 1) / SD_Z;
+    sd_start_kernel<<<blocks_for(n + 1, 256, 16), 256, 0, st>>>(kin, n, (unsigned)dims, (unsigned)nseg, ws.entries,
+                                                                ws.start);
     PYL_LAUNCH_CHECK();
     sd_gather_kernel<SHIFT><<<blocks_for(n, 256, 16), 256, 0, st>>>(pos, w, vin, n, halfcell, ws.spos);
     PYL_LAUNCH_CHECK();
     stage_mark(PYL_STAGE_SORT, false, st);
     stage_mark(PYL_STAGE_DEPOSIT, true, st);
-    const dim3 blk(32, 8), grd((unsigned)((dims + 31) / 32), (unsigned)((dims + 7) / 8), (unsigned)dims);
     const int f = fold ? 1 : 0;
-    const unsigned cap = (unsigned)g_sd_stage_cap.load();
-    if (w) sd_deposit_kernel<MAS, true><<<grd, blk, 0, st>>>(ws.spos, ws.runs, dims, inv, out, scale_h, scale_d, f, cap);
-    else sd_deposit_kernel<MAS, false><<<grd, blk, 0, st>>>(ws.spos, ws.runs, dims, inv, out, scale_h, scale_d, f, cap);
+    if constexpr (MAS == PYL_MAS_NGP) {
+        auto kern = w ? sd_ngp_kernel<true> : sd_ngp_kernel<false>;
+        kern<<<blocks_for(cells, 256, 32), 256, 0, st>>>(ws.spos, kin, ws.start, dims, nseg, cells, out, scale_h, scale_d, f);
+    } else {
+        constexpr int H = MAS - 1;
+        // layers per CTA: SD_CTA_LAYERS, or fewer (each CTA brings its own S-1 halo layers)
+        // until the CTAs are two per SM
+        const unsigned gy = (unsigned)((dims + SDY - H - 1) / (SDY - H)), gx = (unsigned)((dims + SDX - H - 1) / (SDX - H));
+        int zs = SD_CTA_LAYERS;
+        while (zs > 8 && (long long)gx * gy * ((dims + zs - 1) / zs) < 2LL * num_sms()) zs /= 2;
+        constexpr size_t smem = SdShape<MAS>::SMEM;
+        auto kern = w ? sd_deposit_kernel<MAS, true> : sd_deposit_kernel<MAS, false>;
+        PYL_CUDA(ensure_smem(kern, smem));
+        kern<<<dim3((unsigned)((dims + zs - 1) / zs), gy, gx), dim3(SDY, SDX), smem, st>>>(
+            ws.spos, kin, ws.start, dims, nseg, zs, inv, out, scale_h, scale_d, f);
+    }
     PYL_LAUNCH_CHECK();
     stage_mark(PYL_STAGE_DEPOSIT, false, st);
     return PYL_OK;
@@ -668,9 +614,9 @@ int launch_sorted(int mas, const float *pos, const float *w, long long n, float 
 
 }  // namespace pyl
 
+// The deposit stages no particles any more: every limit gives the same sums.
 extern "C" int pyl_sorted_set_stage_limit(int max_particles)
 {
-    PYL_CHECK_ARG(max_particles <= pyl::SDT_CAP, "max_particles above the stage capacity (1024)");
-    pyl::g_sd_stage_cap.store(max_particles < 0 ? pyl::SDT_CAP : max_particles);
+    PYL_CHECK_ARG(max_particles <= 1024, "max_particles above the stage capacity (1024)");
     return PYL_OK;
 }
