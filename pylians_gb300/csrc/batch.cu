@@ -20,61 +20,6 @@
 namespace pyl {
 namespace {
 
-__device__ __forceinline__ float ba_dist(float p, float inv) { return __fmul_rn(p, inv); }
-
-// Support of one coordinate (same arithmetic as mas.cu axis_weights).
-template <int MAS>
-__device__ __forceinline__ int ba_weights(float p, float inv, float *C)
-{
-    const float dist = ba_dist(p, inv);
-    if (MAS == PYL_MAS_NGP) {
-        const float fl = floorf(dist);
-        const float frac = __fsub_rn(dist, fl);
-        int k = __float2int_rz(fl) + (frac >= 0.5f ? 1 : 0);
-        if (dist < -0.5f && frac != 0.5f) k += 1;
-        C[0] = 1.0f;
-        return k;
-    } else if (MAS == PYL_MAS_CIC) {
-        const float t = truncf(dist);
-        const float u = __fsub_rn(dist, t);
-        C[0] = __fsub_rn(1.0f, u);
-        C[1] = u;
-        return __float2int_rz(t);
-    } else if (MAS == PYL_MAS_TSC) {
-        const float fl = floorf(dist);
-        const float frac = __fsub_rn(dist, fl);
-        const float fmn = __fsub_rn(__fadd_rn(fl, frac >= 0.5f ? 1.0f : 0.0f), 2.0f);
-#pragma unroll
-        for (int j = 0; j < 3; j++) {
-            const float diff = fabsf(__fsub_rn(__fadd_rn(fmn, (float)(j + 1)), dist));
-            float c;
-            if (diff < 0.5f) c = __fsub_rn(0.75f, __fmul_rn(diff, diff));
-            else if (diff < 1.5f) { const float t = __fsub_rn(1.5f, diff); c = __fmul_rn(__fmul_rn(0.5f, t), t); }
-            else c = 0.0f;
-            C[j] = c;
-        }
-        return __float2int_rz(fl) - 1 + (frac >= 0.5f ? 1 : 0);
-    } else {
-        const float fl = floorf(dist);
-        const float fmn = __fsub_rn(fl, 2.0f);
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const float d = fabsf(__fsub_rn(__fadd_rn(fmn, (float)(j + 1)), dist));
-            float c;
-            if (d < 1.0f) {
-                const float a = __fmul_rn(__fmul_rn(6.0f, d), d);
-                const float b = __fmul_rn(__fmul_rn(__fmul_rn(3.0f, d), d), d);
-                c = __fdiv_rn(__fadd_rn(__fsub_rn(4.0f, a), b), 6.0f);
-            } else if (d < 2.0f) {
-                const float t = __fsub_rn(2.0f, d);
-                c = __fdiv_rn(__fmul_rn(__fmul_rn(t, t), t), 6.0f);
-            } else c = 0.0f;
-            C[j] = c;
-        }
-        return __float2int_rz(fl) - 1;
-    }
-}
-
 template <int MAS>
 __device__ __forceinline__ void ba_deposit(const float *p, const pyl_batch_real &r, float shift, float *out)
 {
@@ -85,7 +30,7 @@ __device__ __forceinline__ void ba_deposit(const float *p, const pyl_batch_real 
     int idx[3][S];
 #pragma unroll
     for (int a = 0; a < 3; a++) {
-        const int f = ba_weights<MAS>(__fadd_rn(p[a], shift), r.inv, C[a]);
+        const int f = axis_weights<MAS>(__fadd_rn(p[a], shift), r.inv, C[a]);
 #pragma unroll
         for (int j = 0; j < S; j++) idx[a][j] = wrap_index((long long)f + j, dims);
     }

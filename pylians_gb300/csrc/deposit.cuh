@@ -37,6 +37,23 @@ __device__ __forceinline__ int axis_first(float p, float inv)
     return fi - 1;                                        // PCS
 }
 
+// x / 6 correctly rounded, for normal x: the product with the rounded reciprocal and one
+// fused correction of its residual (P. Markstein, IBM J. Res. Dev. 34, 1990).  The weights'
+// numerators are 0 or at least 2^-69.
+__device__ __forceinline__ float sixth(float x)
+{
+    const float q = __fmul_rn(x, 1.0f / 6.0f);
+    return __fmaf_rn(__fmaf_rn(-6.0f, q, x), 1.0f / 6.0f, q);
+}
+
+// Coordinates (in cells) below which the distances to a particle's cells lie where its
+// first cell puts them, so that each weight has one formula.  Past it (and for what is not
+// finite) the weights follow from the distances as they come out.  All float32 coordinates
+// give the same bits either way.  Computing both formulas for every weight, with 24
+// divisions a particle for PCS, bound the deposits' instructions: 512^3 PCS interlaced
+// 10.81 -> 9.49 ms, sorted 256^3 TSC 2.00 -> 1.82 ms.
+constexpr float WEIGHT_FAST = 4194304.0f;
+
 // Per-axis support of one particle coordinate: first cell f (unwrapped) and the
 // S weights of cells f, f+1, ..., f+S-1.  f equals axis_first<MAS>(p, inv).
 template <int MAS>
@@ -58,6 +75,14 @@ __device__ __forceinline__ int axis_weights(float p, float inv, float *C)
         const float frac = __fsub_rn(dist, fl);
         const int mn = __float2int_rz(fl) - 2 + (frac >= 0.5f ? 1 : 0);  // floor(dist - 1.5)
         const float fmn = __fsub_rn(__fadd_rn(fl, frac >= 0.5f ? 1.0f : 0.0f), 2.0f);
+        if (fabsf(dist) < WEIGHT_FAST) {                  // the middle cell within 1/2, the others from 1/2 to 3/2
+            const float d0 = __fsub_rn(dist, __fadd_rn(fmn, 1.0f)), d1 = __fsub_rn(__fadd_rn(fmn, 2.0f), dist);
+            const float t0 = __fsub_rn(1.5f, d0), t2 = __fsub_rn(1.5f, __fsub_rn(__fadd_rn(fmn, 3.0f), dist));
+            C[0] = __fmul_rn(__fmul_rn(0.5f, t0), t0);
+            C[1] = __fsub_rn(0.75f, __fmul_rn(d1, d1));
+            C[2] = __fmul_rn(__fmul_rn(0.5f, t2), t2);
+            return mn + 1;
+        }
 #pragma unroll
         for (int j = 0; j < 3; j++) {
             const float diff = fabsf(__fsub_rn(__fadd_rn(fmn, (float)(j + 1)), dist));
@@ -77,6 +102,18 @@ __device__ __forceinline__ int axis_weights(float p, float inv, float *C)
         const float fl = floorf(dist);
         const int mn = __float2int_rz(fl) - 2;            // floor(dist - 2)
         const float fmn = __fsub_rn(fl, 2.0f);
+        if (fabsf(dist) < WEIGHT_FAST) {                  // distances 1 + u, u, 1 - u, 2 - u of u in [0, 1)
+            const float u = __fsub_rn(dist, fl), v = __fsub_rn(__fadd_rn(fl, 1.0f), dist);
+            const float t0 = __fsub_rn(2.0f, __fsub_rn(dist, __fadd_rn(fmn, 1.0f)));
+            const float t3 = __fsub_rn(2.0f, __fsub_rn(__fadd_rn(fmn, 4.0f), dist));
+            C[0] = sixth(__fmul_rn(__fmul_rn(t0, t0), t0));
+            C[1] = sixth(__fadd_rn(__fsub_rn(4.0f, __fmul_rn(__fmul_rn(6.0f, u), u)),
+                                   __fmul_rn(__fmul_rn(__fmul_rn(3.0f, u), u), u)));
+            C[2] = sixth(__fadd_rn(__fsub_rn(4.0f, __fmul_rn(__fmul_rn(6.0f, v), v)),
+                                   __fmul_rn(__fmul_rn(__fmul_rn(3.0f, v), v), v)));
+            C[3] = sixth(__fmul_rn(__fmul_rn(t3, t3), t3));
+            return mn + 1;
+        }
 #pragma unroll
         for (int j = 0; j < 4; j++) {
             const float d = fabsf(__fsub_rn(__fadd_rn(fmn, (float)(j + 1)), dist));
