@@ -233,6 +233,15 @@ int pyl_pk_bin(const void *dk, const void *dk_interlaced, int n_fields, int64_t 
 int pyl_pk_geometry(int dims, int axis, double *geom, void *workspace, size_t workspace_bytes,
                     void *stream);
 
+/* Host finalisation (Pk_library.pyx:384-421, :740-796): every pointer is HOST memory.
+ * consts: kF, kN^2, fact = (BoxSize/dims^2)^3, pi, (2 pi)^2.  n_cross: -1 for Pk's
+ * results (the first field), else the cross pairs F(F-1)/2 for XPk's (FO = F).  out:
+ * 14 arrays, k1D [nb1-1], N1 [nb1-1], P1 [nb1-1][FO], PX1 [nb1-1][X], kpar [nb2],
+ * kper [nb2], N2 [nb2], P2 [nb2][FO], PX2 [nb2][X], k3D [nb3-1], N3 [nb3-1],
+ * P3 [nb3-1][3][FO], PX3 [nb3-1][3][X], phase [nb3-1] (Pk); those of X NULL for Pk. */
+int pyl_pk_finalize(const double *sums, const double *geom, int dims, int n_fields, int n_cross,
+                    const double *consts, double *const *out);
+
 /* Many one-field spectra of one grid side in one launch (the batched-realization
  * path; no counterpart in the reference, which bins one field per Pk call).  `items`
  * is a DEVICE array of n_items records, each one pyl_pk_bin call with n_fields = 1:

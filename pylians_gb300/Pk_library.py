@@ -19,6 +19,7 @@ Differences: check_number_modes(_2D) raise RuntimeError instead of sys.exit();
 keyword-only `interlaced=` takes the half-cell-shifted grid(s) produced by
 MAS_library.MA(..., interlaced=...).  Inputs may be numpy arrays or CUDA tensors.
 """
+import ctypes
 import math
 import time
 
@@ -140,7 +141,6 @@ def pk_sums_device(dk, dims, axis, mas_list, dk_interlaced=None, out=None, strea
 
 
 def ctypes_int_array(vals):
-    import ctypes
     arr = (ctypes.c_int * len(vals))(*[int(v) for v in vals])
     return ctypes.cast(arr, ctypes.c_void_p), arr
 
@@ -149,47 +149,35 @@ class _Result(object):
     pass
 
 
+_FinalizeConsts, _FinalizeOut = ctypes.c_double * 5, ctypes.c_void_p * 14
+
+
 def finalize_pk(sums, geom, BoxSize, dims, F, cross):
     """Host float64 finalisation: Pk_library.pyx:384-421 (Pk) and :740-796 (XPk)."""
     kF, kN, kmax_par, kmax_per, kmax = frequencies(BoxSize, dims)
-    fact = (BoxSize / dims ** 2) ** 3
+    nb1, nb2, nb3 = kmax_par + 1, (kmax_par + 1) * (kmax_per + 1), kmax + 1
     X = F * (F - 1) // 2
-    s = _split_sums(sums, dims, F)
-    g = _split_geometry(geom, dims)
+    sums = np.ascontiguousarray(sums, dtype=np.float64)
+    geom = np.ascontiguousarray(geom, dtype=np.float64)
+    if sums.size < (3 * nb3 + nb1 + nb2) * (F + X) + nb3 * F or geom.size < 2 * nb1 + nb2 + 2 * nb3:
+        raise ValueError('sums or geometry too short for %d^3 cells and %d fields' % (dims, F))
+    check_number_modes(geom[2 * nb1 + nb2 + nb3:2 * nb1 + nb2 + 2 * nb3], dims)
+    e, fo = np.empty, (F,) if cross else ()
     r = _Result()
-    with np.errstate(divide='ignore', invalid='ignore'):
-        N1 = g['N1'][1:].copy()
-        k1D = (g['K1'][1:] / N1) * kF
-        kmaxper = np.sqrt(kN ** 2 - k1D ** 2)
-        area = (np.pi * kmaxper ** 2 / N1) / (2.0 * np.pi) ** 2
-        P1 = s['P1'][1:] * fact * area[:, None]
-        ip = np.arange(kmax_par + 1)
-        iq = np.arange(kmax_per + 1)
-        kpar = np.zeros((kmax_par + 1) * (kmax_per + 1))
-        kper = np.zeros_like(kpar)
-        idx = (kmax_par + 1) * iq[None, :] + ip[:, None]
-        kpar[idx] = (0.5 * (ip + ip + 1) * kF)[:, None]
-        kper[idx] = (0.5 * (iq + iq + 1) * kF)[None, :]
-        N2 = g['N2'].copy()
-        P2 = s['P2'] * fact / N2[:, None]
-        check_number_modes(g['N3'], dims)
-        N3 = g['N3'][1:].copy()
-        k3D = (g['K3'][1:] / N3) * kF
-        P3 = s['P3'][1:].copy()
-        P3[:, 0] = (P3[:, 0] / N3[:, None]) * fact
-        P3[:, 1] = (P3[:, 1] * 5.0 / N3[:, None]) * fact
-        P3[:, 2] = (P3[:, 2] * 9.0 / N3[:, None]) * fact
-        PH = (s['PH'][1:] / N3[:, None]) * fact
-    r.k1D, r.Nmodes1D = k1D, N1
-    r.kpar, r.kper, r.Nmodes2D = kpar, kper, N2
-    r.k3D, r.Nmodes3D = k3D, N3
+    r.k1D, r.Nmodes1D, r.Pk1D = e(nb1 - 1), e(nb1 - 1), e((nb1 - 1,) + fo)
+    r.kpar, r.kper, r.Nmodes2D, r.Pk2D = e(nb2), e(nb2), e(nb2), e((nb2,) + fo)
+    r.k3D, r.Nmodes3D, r.Pk = e(nb3 - 1), e(nb3 - 1), e((nb3 - 1, 3) + fo)
     if cross:
-        r.Pk1D, r.PkX1D = np.ascontiguousarray(P1[:, :F]), np.ascontiguousarray(P1[:, F:F + X])
-        r.Pk2D, r.PkX2D = np.ascontiguousarray(P2[:, :F]), np.ascontiguousarray(P2[:, F:F + X])
-        r.Pk, r.XPk = np.ascontiguousarray(P3[:, :, :F]), np.ascontiguousarray(P3[:, :, F:F + X])
+        r.PkX1D, r.PkX2D, r.XPk = e((nb1 - 1, X)), e((nb2, X)), e((nb3 - 1, 3, X))
+        x1, x2, x3, phase = r.PkX1D, r.PkX2D, r.XPk, None
     else:
-        r.Pk1D, r.Pk2D = P1[:, 0].copy(), P2[:, 0].copy()
-        r.Pk, r.Pkphase = np.ascontiguousarray(P3[:, :, 0]), PH[:, 0].copy()
+        x1 = x2 = x3 = None
+        r.Pkphase = phase = e(nb3 - 1)
+    out = (r.k1D, r.Nmodes1D, r.Pk1D, x1, r.kpar, r.kper, r.Nmodes2D, r.Pk2D, x2, r.k3D, r.Nmodes3D, r.Pk, x3, phase)
+    consts = _FinalizeConsts(kF, kN ** 2, (BoxSize / dims ** 2) ** 3, np.pi, (2.0 * np.pi) ** 2)
+    _lib.call('pyl_pk_finalize', sums.ctypes.data, geom.ctypes.data, dims, F, X if cross else -1, consts,
+              _FinalizeOut(*[ctypes.addressof(ctypes.c_char.from_buffer(a)) if a is not None and a.size else None
+                             for a in out]))     # a third of the time of a.ctypes.data
     return r
 
 
