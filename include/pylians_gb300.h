@@ -444,12 +444,19 @@ int pyl_wait_probe(unsigned arm_bytes, long long cycles, unsigned *completed, vo
  * pyl_cic_interp replaces MAS_library.CIC_interp (library/MAS_library/MAS_library.pyx:558-599):
  * out[i] = CIC interpolation of grid [dims]^3 at pos[i] (float32 [n][3]), the
  * eight terms added in the reference's order; indices wrap non-negatively.
+ * pyl_cic_interp_slabs gives the same bits from a workspace of
+ * pyl_cic_interp_workspace_size() bytes (16-byte aligned), faster for many particles
+ * in no order on a grid larger than L2; the size is 0 where pyl_cic_interp is the
+ * faster one whatever the order.
  * pyl_pos_redshift_space replaces redshift_space_library.pos_redshift_space
  * (library/redshift_space_library.pyx:29-43): pos[:,axis] += vel[:,axis] *
  * (1+redshift)/Hubble in place, then positions above box_size or below 0 become
  * fmod(pos + box_size, box_size). */
 int pyl_cic_interp(const float *grid, int dims, float box_size, const float *pos, int64_t n, float *out,
                    void *stream);
+size_t pyl_cic_interp_workspace_size(int dims, int64_t n);
+int pyl_cic_interp_slabs(const float *grid, int dims, float box_size, const float *pos, int64_t n, float *out,
+                         void *workspace, size_t workspace_bytes, void *stream);
 int pyl_pos_redshift_space(float *pos, const float *vel, int64_t n, float box_size, float hubble,
                            float redshift, int axis, void *stream);
 

@@ -121,6 +121,16 @@ def MA(pos, number, BoxSize, MAS='CIC', W=None, verbose=False, renormalize_2D=Tr
         print('Time taken = %.3f seconds\n' % (time.time() - start))
 
 
+def _interp_workspace(grid, n):
+    """Scratch for the interpolation by slabs, the call's own (concurrent calls on several
+    streams share nothing); None where it brings nothing or the memory is not there."""
+    nbytes = _lib.load().pyl_cic_interp_workspace_size(grid.shape[0], n)
+    try:
+        return torch.empty(nbytes, dtype=torch.uint8, device=grid.device) if nbytes else None
+    except torch.cuda.OutOfMemoryError:
+        return None
+
+
 def CIC_interp(density, BoxSize, pos, den):
     """MAS_library.CIC_interp: den[i] <- CIC interpolation of the 3D density grid at
     pos[i] (the eight corner terms added in the reference's order).  numpy arrays are
@@ -133,8 +143,13 @@ def CIC_interp(density, BoxSize, pos, den):
         raise ValueError('density must be a cubic 3D grid')
     if dpos.dim() != 2 or dpos.shape[1] != 3 or dden.dim() != 1 or dden.shape[0] != dpos.shape[0]:
         raise ValueError('pos must be (N,3) and den (N,)')
-    _lib.call('pyl_cic_interp', ptr(dgrid), dgrid.shape[0], float(BoxSize), ptr(dpos), dpos.shape[0],
-              ptr(dden), stream_ptr())
+    ws = _interp_workspace(dgrid, dpos.shape[0])
+    if ws is None:
+        _lib.call('pyl_cic_interp', ptr(dgrid), dgrid.shape[0], float(BoxSize), ptr(dpos), dpos.shape[0],
+                  ptr(dden), stream_ptr())
+    else:
+        _lib.call('pyl_cic_interp_slabs', ptr(dgrid), dgrid.shape[0], float(BoxSize), ptr(dpos), dpos.shape[0],
+                  ptr(dden), ptr(ws), ws.numel(), stream_ptr())
     if is_torch(den):
         if not den.is_cuda:
             den.copy_(dden.cpu())

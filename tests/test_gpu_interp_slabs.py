@@ -1,0 +1,55 @@
+"""Interpolation by slabs against cic_interp_kernel (one particle after the other): the
+same bits, for one to 256 slabs, particle counts at the edges of its tiles (4096) and of
+its passes (2^25), particles in no order, sorted along x and along z, outside the box and
+not finite."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+BOX = 1000.0
+
+
+def _both(g, pos):
+    import pylians_gb300.build as b
+    b.build()
+    from pylians_gb300 import _lib
+    from pylians_gb300._device import ptr, stream_ptr
+    n, dims = pos.shape[0], g.shape[0]
+    a, c = (torch.full((n + 1,), 7.0, device='cuda') for _ in range(2))
+    ws = torch.empty(18 * 4096 * min(8192, (n + 4095) // 4096) + 4 * 514 * 8192, dtype=torch.uint8, device='cuda')
+    _lib.call('pyl_cic_interp', ptr(g), dims, BOX, ptr(pos), n, ptr(a), stream_ptr())
+    _lib.call('pyl_cic_interp_slabs', ptr(g), dims, BOX, ptr(pos), n, ptr(c), ptr(ws), ws.numel(), stream_ptr())
+    assert torch.equal(a.view(torch.int32), c.view(torch.int32))
+    with pytest.raises(_lib.PylError):
+        _lib.call('pyl_cic_interp_slabs', ptr(g), dims, BOX, ptr(pos), n, ptr(c), ptr(ws), 16, stream_ptr())
+
+
+@pytest.mark.parametrize('order', ['none', 'x', 'z'])
+@pytest.mark.parametrize('dims,n', [(1, 5000), (7, 1), (64, 4095), (163, 4096), (163, 4097), (300, 3 * 4096 + 5),
+                                    (300, 300000), (601, 100000), (1024, 1000000), (64, 2 ** 25 + 4099)])
+def test_slabs_same_bits(dims, n, order):
+    torch.manual_seed(n)
+    g = torch.randn((dims,) * 3, device='cuda')
+    pos = torch.rand(n, 3, device='cuda') * BOX
+    if order != 'none':
+        pos = pos[torch.argsort(pos[:, 'xyz'.index(order)])].contiguous()
+    k = min(n, 9)
+    pos[:k, 0] = torch.tensor([0.0, BOX, -1.0, 3.5 * BOX, float('nan'), float('inf'), -float('inf'), -1e30, BOX - 1e-4],
+                              device='cuda')[:k]
+    _both(g, pos)
+
+
+def test_public_call_takes_slabs():
+    import pylians_gb300.MAS_library as MASL
+    from pylians_gb300 import _lib
+    from pylians_gb300._device import ptr, stream_ptr
+    dims, n = 400, 2 ** 23
+    assert _lib.load().pyl_cic_interp_workspace_size(dims, n) > 0
+    assert _lib.load().pyl_cic_interp_workspace_size(dims, n - 1) == 0
+    torch.manual_seed(0)
+    g, pos = torch.randn((dims,) * 3, device='cuda'), torch.rand(n, 3, device='cuda') * BOX
+    a, c = torch.empty(n, device='cuda'), torch.empty(n, device='cuda')
+    MASL.CIC_interp(g, BOX, pos, a)
+    _lib.call('pyl_cic_interp', ptr(g), dims, BOX, ptr(pos), n, ptr(c), stream_ptr())
+    assert torch.equal(a, c)
