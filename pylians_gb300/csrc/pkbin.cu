@@ -64,6 +64,28 @@ __device__ __forceinline__ T seg_sum(T v, int start)
     return v;
 }
 
+// The same sums, bit for bit, of N values at once, for the lanes of keys other than
+// KEY_NONE.  Steps that no segment reaches are left out (about half of them): bit i of the
+// mask is set where lane i and the 1, 2, 4, 8, 16 lanes before it are one segment.  Two
+// fields of 512^3, axis 2: 1967 us with all five steps, 1601 so; three of 256^3, axis 0: 367
+// and 290.
+template <int N>
+__device__ __forceinline__ void seg_sums(float (&v)[N], int start, int key)
+{
+    const int lane = threadIdx.x & 31;
+    unsigned more = __ballot_sync(FULL, lane != start && key != KEY_NONE);
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        if (!more) break;
+#pragma unroll
+        for (int c = 0; c < N; c++) {
+            const float y = __shfl_up_sync(FULL, v[c], o);
+            if (lane - o >= start) v[c] += y;
+        }
+        more &= more << o;
+    }
+}
+
 struct BinArgs {
     const float2 *dk, *dk2;
     long long fstride;
@@ -265,35 +287,56 @@ __global__ void __launch_bounds__(256) pk_bin_kernel(BinArgs a)
             const Seg s3 = seg_of(ki);
             float *b3 = acc3 + (ki == KEY_NONE ? 0 : ki) * slots3;
             const bool t3 = s3.tail && ki != KEY_NONE;
-#pragma unroll
-            for (int c = 0; c < C; c++) {
-                const float v0 = seg_sum(val[c], s3.start);
-                const float v2 = seg_sum(val[c] * l2, s3.start);
-                const float v4 = seg_sum(val[c] * l4, s3.start);
-                if (t3) {
-                    atomicAdd(b3 + 3 * c, v0);
-                    atomicAdd(b3 + 3 * c + 1, v2);
-                    atomicAdd(b3 + 3 * c + 2, v4);
-                }
-            }
+            float sq[F];
 #pragma unroll
             for (int f = 0; f < F; f++) {
                 const float p2 = val[f];
                 // phase = atan2(Re d, |d|) = atan(Re d / |d|), |Re d / |d|| <= 1
                 const float phase = p2 > 0.0f ? atan_unit(re[f] * rsqrtf(p2)) : 0.0f;
-                const float vph = seg_sum(phase * phase, s3.start);
-                if (t3) atomicAdd(b3 + 3 * C + f, vph);
+                sq[f] = phase * phase;
+            }
+            if constexpr (F <= 2) {
+                float v[3 * C + F];
+#pragma unroll
+                for (int c = 0; c < C; c++) {
+                    v[3 * c] = val[c];
+                    v[3 * c + 1] = val[c] * l2;
+                    v[3 * c + 2] = val[c] * l4;
+                }
+#pragma unroll
+                for (int f = 0; f < F; f++) v[3 * C + f] = sq[f];
+                seg_sums(v, s3.start, ki);
+                if (t3)
+#pragma unroll
+                    for (int c = 0; c < 3 * C + F; c++) atomicAdd(b3 + c, v[c]);
+            } else {                                        // fewer registers
+#pragma unroll
+                for (int c = 0; c < C; c++) {
+                    float v[3] = {val[c], val[c] * l2, val[c] * l4};
+                    seg_sums(v, s3.start, ki);
+                    if (t3)
+#pragma unroll
+                        for (int i = 0; i < 3; i++) atomicAdd(b3 + 3 * c + i, v[i]);
+                }
+                seg_sums(sq, s3.start, ki);
+                if (t3)
+#pragma unroll
+                    for (int f = 0; f < F; f++) atomicAdd(b3 + 3 * C + f, sq[f]);
             }
             if (AXIS != 2) {
                 // 2D by k_per (shared memory), 1D by the plane's k_par (registers)
                 const Seg s2 = seg_of(valid ? kper : KEY_NONE);
                 const bool t2 = s2.tail && valid;
+                float v[C];
 #pragma unroll
                 for (int c = 0; c < C; c++) {
-                    const float v = seg_sum(val[c], s2.start);
-                    if (t2) atomicAdd(acc2 + kper * C + c, v);
+                    v[c] = val[c];
                     if (in1d) r1[c] += val[c];
                 }
+                seg_sums(v, s2.start, valid ? kper : KEY_NONE);
+                if (t2)
+#pragma unroll
+                    for (int c = 0; c < C; c++) atomicAdd(acc2 + kper * C + c, v[c]);
             } else if (a.warp_arrays) {
                 if (valid) {
 #pragma unroll
