@@ -32,6 +32,7 @@ constexpr int MAX_FIELDS = 4;
 constexpr int NW = 8;                    // warps per CTA (256 threads)
 constexpr unsigned FULL = 0xffffffffu;
 constexpr int KEY_NONE = 0x7fffffff;
+constexpr int RING_ROWS_PER_CTA = 256;
 
 struct Seg {
     int start;
@@ -97,6 +98,7 @@ struct BinArgs {
     const unsigned *rows;  // axis 2: row ids (kxx*dims + kyy) sorted by k_per ring
     int chunks;            // axis 0/1: CTAs per plane
     int rows_per_cta;      // axis 2: table entries per CTA
+    int low_ctas;          // axis 2, pk_bin_kernel: first CTAs, of RING_ROWS_PER_CTA entries each
     int warp_arrays;       // axis 2: per-warp kz arrays in shared memory
     float *part;           // one field: per-CTA partial sums in global memory (null: shared memory)
     int part_stride;       // floats per CTA: 3D bins x 4, then k_per bins (axes 0/1)
@@ -145,9 +147,12 @@ __device__ __forceinline__ RowIter row_iter(const BinArgs &a, int warp)
     } else {
         it.plane = 0;
         const long long total = (long long)dims * dims;
-        const long long b = (long long)blockIdx.x * a.rows_per_cta;
-        const long long e = min(total, b + a.rows_per_cta);
-        const int L = (a.rows_per_cta + NW - 1) / NW;
+        const int low = a.low_ctas - (int)blockIdx.x;       // > 0: one of the first rows' CTAs
+        const int per = low > 0 ? RING_ROWS_PER_CTA : a.rows_per_cta;
+        const long long b = low > 0 ? (long long)blockIdx.x * per
+                                    : (long long)a.low_ctas * RING_ROWS_PER_CTA - (long long)low * per;
+        const long long e = min(total, b + per);
+        const int L = (per + NW - 1) / NW;
         const long long wb = b + (long long)warp * L;
         it.first = (int)wb;
         it.step = 1;
@@ -1056,8 +1061,26 @@ inline int plane_chunks(int dims)
     return chunks;
 }
 
-constexpr int RING_ROWS_PER_CTA = 256;
-constexpr size_t SMEM_LIMIT = 200 * 1024;
+constexpr int RING_ROWS_MIN = 32, RING_LOW_CTAS = 4;
+constexpr size_t SMEM_LIMIT = 200 * 1024, SMEM_SM = 228 * 1024;
+
+// Rows of the ring table for a CTA: at most RING_ROWS_PER_CTA, as few as fill whole waves of
+// the CTAs resident at once, but RING_ROWS_MIN for each CTA's tables, zeroing and flushes.
+// 256 rows for all left most SMs idle at small sides and 2.2 waves at 512^3, two fields.
+// us of the bin kernels, 256 rows and now: P(k) 64^3 79 and 13, 128^3 95 and 18, 512^3 279 and
+// 203; XPk two fields 128^3 155 and 93, 512^3 1601 and 1346; four of 200^3 612 and 370.
+inline long long ring_waves(long long rows, int resident)
+{
+    const long long slots = (long long)resident * num_sms() * RING_ROWS_PER_CTA;
+    return (rows + slots - 1) / slots;
+}
+
+inline int ring_rows_per_cta(long long rows, int resident)
+{
+    const long long ctas = ring_waves(rows, resident) * resident * num_sms();
+    return (int)std::max<long long>(RING_ROWS_MIN, (rows + ctas - 1) / ctas);
+}
+constexpr int SEQ_RESIDENT = 4;          // pk_bin_seq_kernel: 64 registers
 
 struct SeqPart {
     unsigned blocks;
@@ -1078,7 +1101,8 @@ inline int sym_chunks(int dims)
 inline SeqPart seq_part(const PkDims &d, int axis)
 {
     SeqPart p;
-    p.blocks = axis == 2 ? (unsigned)((ring_rows(d, true) + RING_ROWS_PER_CTA - 1) / RING_ROWS_PER_CTA)
+    const int rpc = axis == 2 ? ring_rows_per_cta(ring_rows(d, true), SEQ_RESIDENT) : 0;
+    p.blocks = axis == 2 ? (unsigned)((ring_rows(d, true) + rpc - 1) / rpc)
                          : (unsigned)(sym_groups(d.dims) * sym_chunks(d.dims));
     p.stride = (d.nb3 * 4 + (axis == 2 ? 0 : d.kmax_per + 1) + 3) & ~3;
     p.bytes = align256(sizeof(float) * (size_t)p.blocks * p.stride);
@@ -1146,6 +1170,7 @@ extern "C" int pyl_pk_bin(const void *dk, const void *dk_interlaced, int n_field
     a.part = nullptr;
     a.part_stride = 0;
     a.items = nullptr;
+    a.low_ctas = 0;
     for (int f = 0; f < MAX_FIELDS; f++) {
         a.mas_p[f] = f < n_fields ? host_mas_p[f] : 0;
         PYL_CHECK_ARG(a.mas_p[f] >= 0 && a.mas_p[f] <= 4, "MAS exponent must be 0..4");
@@ -1171,10 +1196,17 @@ extern "C" int pyl_pk_bin(const void *dk, const void *dk_interlaced, int n_field
         int rc = build_rings(d, w, seq, st);
         if (rc) return rc;
         a.rows = w.rows;
-        a.rows_per_cta = RING_ROWS_PER_CTA;
+        // pk_bin_kernel: 64 registers, or what its shared memory leaves
+        const size_t smem = sizeof(float) * (size_t)bin_smem(d, a.F, a.C, axis, inter, warp_arrays).total;
+        const int resident = seq ? SEQ_RESIDENT : (int)std::min<size_t>(4, std::max<size_t>(1, SMEM_SM / (smem + 1024)));
+        a.rows_per_cta = ring_rows_per_cta(ring_rows(d, seq), resident);
         a.chunks = 1;
         a.warp_arrays = warp_arrays;
-        blocks = (unsigned)((ring_rows(d, seq) + RING_ROWS_PER_CTA - 1) / RING_ROWS_PER_CTA);
+        // several waves: the first rows, whose bins hold few modes, in CTAs of the full length,
+        // so that few warps share a bin's sum
+        if (!seq && ring_waves(ring_rows(d, false), resident) > 1) a.low_ctas = RING_LOW_CTAS;
+        const long long rest = ring_rows(d, seq) - (long long)a.low_ctas * RING_ROWS_PER_CTA;
+        blocks = (unsigned)(a.low_ctas + (rest + a.rows_per_cta - 1) / a.rows_per_cta);
     } else {
         a.rows_per_cta = 0;
         a.warp_arrays = 0;
@@ -1273,7 +1305,7 @@ inline BatchPart batch_part(const PkDims &d, int axis, int n_items)
         b.blocks = (unsigned)(G * c);
     } else {
         const long long rows = ring_rows(d, true);
-        int rpc = RING_ROWS_PER_CTA;
+        int rpc = ring_rows_per_cta(rows, SEQ_RESIDENT);
         while (rpc < 16 * RING_ROWS_PER_CTA && ((rows + 2 * rpc - 1) / (2 * rpc)) * n_items >= target) rpc *= 2;
         b.chunks = 1;
         b.rows_per_cta = rpc;
@@ -1386,6 +1418,7 @@ extern "C" int pyl_pk_geometry(int dims, int axis, double *geom, void *workspace
     a.part = nullptr;
     a.part_stride = 0;
     a.items = nullptr;
+    a.low_ctas = 0;
     for (int f = 0; f < MAX_FIELDS; f++) a.mas_p[f] = 0;
     unsigned blocks;
     if (axis == 2) {
