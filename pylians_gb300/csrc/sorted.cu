@@ -1,21 +1,18 @@
 // SORTED strategy of pyl_ma / pyl_ma_overdensity: a deterministic mass
 // assignment built from a sort by cell key and a per-cell segmented reduction.
 //
-//   1. key kernel: every particle's base cell (the first cell of its support on
-//      each axis, wrapped; MAS_library.pyx:123-545 index arithmetic) as a 32-bit
-//      key (ix*dims + iy)*dims + iz, value = particle index.
-//   2. stable LSD radix sort of (key, index), 8-bit digits: per-tile digit
-//      histograms, one exclusive scan over [digit][tile], and a scatter that
-//      ranks each tile's keys stably (warp match + per-warp digit counts) and
-//      stages them in shared memory so global writes are coalesced.  Equal keys
-//      keep increasing particle index.
-//   3. the particles' positions (and weights) gathered into sorted order, and a table of
-//      where each column (ix, iy) and every SD_Z cells along it start there.
+//   1. every particle's base cell (the first cell of its support on each axis, wrapped;
+//      MAS_library.pyx:123-545 index arithmetic) gives a 32-bit key (ix*dims + iy)*dims + iz.
+//   2. stable LSD radix sort by key, 8-bit digits, of the particles themselves: per-tile
+//      digit histograms, one exclusive scan over [digit][tile], and a scatter that
+//      ranks each tile's records stably (warp ballots + per-warp digit counts) and
+//      writes them in digit order, coalesced.  Equal keys keep increasing particle index.
+//   3. a table of where each column (ix, iy) and every SD_Z cells along it start.
 //   4. deposit (sd_deposit_kernel): a thread walks a base column (ix, iy) along z and
 //      keeps the S^3 sums that its particles add to, S output layers of S x S columns,
 //      in registers; at every z the layer that no later particle reaches is exchanged
 //      through shared memory and each output cell adds its S^2 base columns' values.
-//      The interlaced grid runs steps 1-4 again on the shifted positions (its own sort).
+//      The interlaced grid runs all steps again on the shifted positions (its own sort).
 //      No atomics: every cell's sum has one fixed order (base columns by (l, m), within
 //      a column particles by z and index), so the grid is bit-reproducible whatever the
 //      launch configuration; NGP adds each cell's particles in index order onto the
@@ -32,9 +29,9 @@
 namespace pyl {
 namespace {
 
-constexpr int RS_THREADS = 256;
-constexpr int RS_ITEMS = 16;
-constexpr int RS_TILE = RS_THREADS * RS_ITEMS;       // 4096 keys per tile
+constexpr int RS_THREADS = 512;
+constexpr int RS_ITEMS = 8;
+constexpr int RS_TILE = RS_THREADS * RS_ITEMS;       // 4096 records per tile
 constexpr int RS_WARPS = RS_THREADS / 32;
 constexpr int SCAN_THREADS = 1024;
 constexpr int SCAN_ITEMS = 4;
@@ -57,45 +54,73 @@ __device__ __forceinline__ int sd_first(float p, float inv)
     return fi - 1;
 }
 
-// ---- 1. keys --------------------------------------------------------------
-// SHIFT: the half-cell-shifted grid's pass, on positions p + halfcell (the
-// float32 sum the other strategies form for the interlaced grid).
-template <int MAS, bool SHIFT>
-__global__ void __launch_bounds__(256) sd_key_kernel(const float *__restrict__ pos, long long n, float inv,
-                                                     float halfcell, int dims, unsigned *__restrict__ keys,
-                                                     unsigned *__restrict__ vals)
+// ---- 1. records and keys ------------------------------------------------------
+// A record is (x, y, z, weight), or without weights (x, y, z, key's bits): the key then
+// needs no second computation.  The first pass forms them from the caller's arrays, on
+// positions p + halfcell for the half-cell-shifted grid (SHIFT: the float32 sum the other
+// strategies form for the interlaced grid).
+struct RsSource {
+    const float *pos, *w;
+    const float4 *rec;
+    float inv, halfcell;
+    int dims;
+};
+
+template <int MAS>
+__device__ __forceinline__ int sd_cell(float p, float inv, int dims)
 {
-    const long long stride = (long long)gridDim.x * blockDim.x;
+    return wrap_index(sd_first<MAS>(p, inv), dims);
+}
+
+template <int MAS>
+__device__ __forceinline__ unsigned sd_key(const float4 &r, float inv, int dims)
+{
     const unsigned d = (unsigned)dims;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-        float p[3] = {__ldg(pos + 3 * i), __ldg(pos + 3 * i + 1), __ldg(pos + 3 * i + 2)};
-        if (SHIFT)
-            for (int a = 0; a < 3; a++) p[a] = __fadd_rn(p[a], halfcell);
-        const unsigned cx = (unsigned)wrap_index(sd_first<MAS>(p[0], inv), dims);
-        const unsigned cy = (unsigned)wrap_index(sd_first<MAS>(p[1], inv), dims);
-        const unsigned cz = (unsigned)wrap_index(sd_first<MAS>(p[2], inv), dims);
-        keys[i] = (cx * d + cy) * d + cz;
-        vals[i] = (unsigned)i;
+    return ((unsigned)sd_cell<MAS>(r.x, inv, dims) * d + (unsigned)sd_cell<MAS>(r.y, inv, dims)) * d +
+           (unsigned)sd_cell<MAS>(r.z, inv, dims);
+}
+
+template <int MAS, bool FIRST, bool SHIFT, bool WEIGHTED>
+__device__ __forceinline__ float4 rs_record(const RsSource &s, long long i, unsigned &key)
+{
+    float4 r;
+    if (FIRST) {
+        r = make_float4(__ldg(s.pos + 3 * i), __ldg(s.pos + 3 * i + 1), __ldg(s.pos + 3 * i + 2),
+                        WEIGHTED ? __ldg(s.w + i) : 0.0f);
+        if (SHIFT) {
+            r.x = __fadd_rn(r.x, s.halfcell);
+            r.y = __fadd_rn(r.y, s.halfcell);
+            r.z = __fadd_rn(r.z, s.halfcell);
+        }
+    } else {
+        r = __ldg(s.rec + i);
     }
+    key = FIRST || WEIGHTED ? sd_key<MAS>(r, s.inv, s.dims) : __float_as_uint(r.w);
+    if (FIRST && !WEIGHTED) r.w = __uint_as_float(key);
+    return r;
 }
 
 // ---- 2. radix sort ----------------------------------------------------------
 // Per-tile histogram of one digit, stored digit-major: hist[digit * tiles + tile].
-__global__ void __launch_bounds__(RS_THREADS) rs_hist_kernel(const unsigned *__restrict__ keys, long long n,
-                                                             int shift, unsigned tiles,
+template <int MAS, bool FIRST, bool SHIFT, bool WEIGHTED>
+__global__ void __launch_bounds__(RS_THREADS) rs_hist_kernel(RsSource src, long long n, int shift, unsigned tiles,
                                                              unsigned *__restrict__ hist)
 {
     __shared__ unsigned h[256];
-    h[threadIdx.x] = 0u;
+    if (threadIdx.x < 256) h[threadIdx.x] = 0u;
     __syncthreads();
     const long long base = (long long)blockIdx.x * RS_TILE;
 #pragma unroll 4
     for (int r = 0; r < RS_ITEMS; r++) {
         const long long i = base + r * RS_THREADS + threadIdx.x;
-        if (i < n) atomicAdd(&h[(keys[i] >> shift) & 255u], 1u);
+        if (i < n) {
+            unsigned key;
+            rs_record<MAS, FIRST, SHIFT, WEIGHTED>(src, i, key);
+            atomicAdd(&h[(key >> shift) & 255u], 1u);
+        }
     }
     __syncthreads();
-    hist[(long long)threadIdx.x * tiles + blockIdx.x] = h[threadIdx.x];
+    if (threadIdx.x < 256) hist[(long long)threadIdx.x * tiles + blockIdx.x] = h[threadIdx.x];
 }
 
 // Exclusive scan of a block of SCAN_THREADS values (one per thread); returns the
@@ -185,79 +210,98 @@ __global__ void __launch_bounds__(SCAN_THREADS) scan_apply_kernel(unsigned *__re
 }
 
 // Stable scatter of one tile by one digit.  Warp w holds the tile's elements
-// w*512 .. w*512+511 (round r, lane l: element w*512 + r*32 + l), so the order
+// w*256 .. w*256+255 (round r, lane l: element w*256 + r*32 + l), so the order
 // (warp, round, lane) is the tile's order.  Each warp ranks its elements with
-// its own digit counters (a match_any per round, no block barrier), one block
-// scan turns the tile's digit counts into each digit's first staging slot and
-// each warp's first slot within it, and the tile is staged in digit order in
-// shared memory before the coalesced write.
-__global__ void __launch_bounds__(RS_THREADS) rs_scatter_kernel(
-    const unsigned *__restrict__ kin, const unsigned *__restrict__ vin, long long n, int shift, unsigned tiles,
-    const unsigned *__restrict__ goff, unsigned *__restrict__ kout, unsigned *__restrict__ vout)
+// its own digit counters (no block barrier), one block scan turns the tile's digit counts
+// into each digit's first slot and each warp's first slot within it, and the records go
+// from shared memory to global in digit order, coalesced.
+// Moves the records, not (key, index) pairs: at 256^3 particles a pass of pairs took 193 us
+// (two CTAs per SM of 16 records a thread in registers, a match_any per 32) and the positions'
+// gather at the end 294; a pass of records takes 135 us, the first, which forms the keys,
+// 195, at 536 and 470 MB: bound by latency at 32 warps per SM, half of them at barriers.
+struct RsSmem {
+    float4 rec[RS_TILE];
+    unsigned short place[RS_TILE];           // element in each slot
+    unsigned char digit[RS_TILE];            // its digit
+    unsigned short wc[RS_WARPS][256];        // a warp's count of each digit, then its first slot
+    unsigned start[256];                     // first slot of each digit
+    unsigned gbase[256];                     // global position of the digit's first element
+    unsigned ws[32];
+};
+
+template <int MAS, bool FIRST, bool SHIFT, bool WEIGHTED>
+__global__ void __launch_bounds__(RS_THREADS, 2) rs_scatter_kernel(RsSource src, long long n, int shift, unsigned tiles,
+                                                                   const unsigned *__restrict__ goff,
+                                                                   float4 *__restrict__ out)
 {
-    constexpr int PER_WARP = RS_ITEMS * 32;
-    __shared__ unsigned sk[RS_TILE], sv[RS_TILE];
-    __shared__ unsigned wc[RS_WARPS][256];   // a warp's count of each digit, then its first slot
-    __shared__ unsigned start[256];          // first staging slot of each digit
-    __shared__ unsigned gbase[256];          // global position of the digit's first element
-    __shared__ unsigned ws[32];
+    extern __shared__ float4 rs_raw[];
+    RsSmem &sm = *reinterpret_cast<RsSmem *>(rs_raw);
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const long long tile0 = (long long)blockIdx.x * RS_TILE;
-    const long long base = tile0 + (long long)warp * PER_WARP;
-    for (int i = lane; i < 256; i += 32) wc[warp][i] = 0u;
-    unsigned dg[RS_ITEMS], key[RS_ITEMS], val[RS_ITEMS], rk[RS_ITEMS];
+    const int base = warp * RS_ITEMS * 32 + lane;            // the thread's elements: base + 32 r
+    const int cnt = (int)min((long long)RS_TILE, n - tile0);
+    for (int i = lane; i < 256; i += 32) sm.wc[warp][i] = 0;
+    unsigned dg[RS_ITEMS], rk[RS_ITEMS];
 #pragma unroll
     for (int r = 0; r < RS_ITEMS; r++) {
-        const long long i = base + r * 32 + lane;
-        key[r] = i < n ? kin[i] : 0u;
-        val[r] = i < n ? vin[i] : 0u;
-        dg[r] = i < n ? ((key[r] >> shift) & 255u) : 256u;
+        const int i = base + r * 32;
+        dg[r] = 256u;
+        if (i < cnt) {
+            unsigned key;
+            sm.rec[i] = rs_record<MAS, FIRST, SHIFT, WEIGHTED>(src, tile0 + i, key);
+            dg[r] = (key >> shift) & 255u;
+        }
     }
     __syncwarp();
     const unsigned lt = (1u << lane) - 1u;
 #pragma unroll
     for (int r = 0; r < RS_ITEMS; r++) {
         const unsigned d = dg[r];
-        const unsigned peers = __match_any_sync(0xffffffffu, d);
+        unsigned peers = __ballot_sync(0xffffffffu, d < 256u);   // lanes past the end matter to none before it
+#pragma unroll
+        for (int b = 0; b < 8; b++) {
+            const bool one = (d >> b) & 1u;
+            const unsigned v = __ballot_sync(0xffffffffu, one);
+            peers &= one ? v : ~v;
+        }
         const unsigned lrank = __popc(peers & lt);
-        const unsigned before = d < 256u ? wc[warp][d] : 0u;
+        const unsigned before = d < 256u ? sm.wc[warp][d] : 0u;
         __syncwarp();
-        if (lrank == 0u && d < 256u) wc[warp][d] = before + (unsigned)__popc(peers);
+        if (lrank == 0u && d < 256u) sm.wc[warp][d] = (unsigned short)(before + __popc(peers));
         __syncwarp();
         rk[r] = before + lrank;
     }
     __syncthreads();
-    // thread t = digit t: the tile's count, its first slot, each warp's first slot
+    // thread t < 256 = digit t: the tile's count, its first slot, each warp's first slot
     unsigned c = 0u;
+    if (t < 256)
 #pragma unroll
-    for (int w = 0; w < RS_WARPS; w++) c += wc[w][t];
-    const unsigned s0 = block_excl_scan(c, ws, nullptr);
-    start[t] = s0;
-    gbase[t] = goff[(long long)t * tiles + blockIdx.x];
-    unsigned run = s0;
+        for (int w = 0; w < RS_WARPS; w++) c += sm.wc[w][t];
+    const unsigned s0 = block_excl_scan(c, sm.ws, nullptr);
+    if (t < 256) {
+        sm.start[t] = s0;
+        sm.gbase[t] = goff[(long long)t * tiles + blockIdx.x];
+        unsigned run = s0;
 #pragma unroll
-    for (int w = 0; w < RS_WARPS; w++) {
-        const unsigned v = wc[w][t];
-        wc[w][t] = run;
-        run += v;
+        for (int w = 0; w < RS_WARPS; w++) {
+            const unsigned v = sm.wc[w][t];
+            sm.wc[w][t] = (unsigned short)run;
+            run += v;
+        }
     }
     __syncthreads();
 #pragma unroll
     for (int r = 0; r < RS_ITEMS; r++) {
         if (dg[r] < 256u) {
-            const unsigned slot = wc[warp][dg[r]] + rk[r];
-            sk[slot] = key[r];
-            sv[slot] = val[r];
+            const unsigned slot = sm.wc[warp][dg[r]] + rk[r];
+            sm.place[slot] = (unsigned short)(base + r * 32);
+            sm.digit[slot] = (unsigned char)dg[r];
         }
     }
     __syncthreads();
-    const unsigned cnt = (unsigned)min((long long)RS_TILE, n - tile0);
-    for (unsigned p = t; p < cnt; p += RS_THREADS) {
-        const unsigned k = sk[p];
-        const unsigned d = (k >> shift) & 255u;
-        const unsigned g = gbase[d] + (p - start[d]);
-        kout[g] = k;
-        vout[g] = sv[p];
+    for (int p = t; p < cnt; p += RS_THREADS) {
+        const unsigned d = sm.digit[p];
+        out[sm.gbase[d] + ((unsigned)p - sm.start[d])] = sm.rec[sm.place[p]];
     }
 }
 
@@ -266,35 +310,20 @@ constexpr int SD_Z = 8;           // cells along z of a segment
 
 // start[t] = first sorted particle with key >= (t / nseg) * dims + (t % nseg) * SD_Z, for
 // t = 0 .. dims^2 * nseg (the last entry: n).
-__global__ void __launch_bounds__(256) sd_start_kernel(const unsigned *__restrict__ keys, long long n, unsigned dims,
-                                                       unsigned nseg, long long entries, unsigned *__restrict__ start)
+template <int MAS, bool WEIGHTED>
+__global__ void __launch_bounds__(256) sd_start_kernel(RsSource src, long long n, unsigned nseg, long long entries,
+                                                       unsigned *__restrict__ start)
 {
     const long long stride = (long long)gridDim.x * blockDim.x;
+    const unsigned dims = (unsigned)src.dims;
     for (long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x; j <= n; j += stride) {
         // entries after the previous particle's segment, up to this one's
-        long long t = j == 0 ? 0 : (long long)(keys[j - 1] / dims) * nseg + keys[j - 1] % dims / SD_Z + 1;
-        const long long e = j == n ? entries : (long long)(keys[j] / dims) * nseg + keys[j] % dims / SD_Z;
+        unsigned a = 0, b = 0;
+        if (j > 0) rs_record<MAS, false, false, WEIGHTED>(src, j - 1, a);
+        if (j < n) rs_record<MAS, false, false, WEIGHTED>(src, j, b);
+        long long t = j == 0 ? 0 : (long long)(a / dims) * nseg + a % dims / SD_Z + 1;
+        const long long e = j == n ? entries : (long long)(b / dims) * nseg + b % dims / SD_Z;
         for (; t <= e; t++) start[t] = (unsigned)j;
-    }
-}
-
-// ---- 3. positions in sorted order -------------------------------------------
-template <bool SHIFT>
-__global__ void __launch_bounds__(256) sd_gather_kernel(const float *__restrict__ pos, const float *__restrict__ w,
-                                                        const unsigned *__restrict__ vals, long long n,
-                                                        float halfcell, float4 *__restrict__ spos)
-{
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x; j < n; j += stride) {
-        const long long i = vals[j];
-        float4 p = make_float4(__ldg(pos + 3 * i), __ldg(pos + 3 * i + 1), __ldg(pos + 3 * i + 2),
-                               w ? __ldg(w + i) : 1.0f);
-        if (SHIFT) {
-            p.x = __fadd_rn(p.x, halfcell);
-            p.y = __fadd_rn(p.y, halfcell);
-            p.z = __fadd_rn(p.z, halfcell);
-        }
-        spos[j] = p;
     }
 }
 
@@ -323,8 +352,8 @@ struct SdShape {
 
 template <int MAS, bool WEIGHTED>
 __global__ void __launch_bounds__(SDX * SDY, MAS == PYL_MAS_PCS ? 1 : 2) sd_deposit_kernel(
-    const float4 *__restrict__ spos, const unsigned *__restrict__ keys, const unsigned *__restrict__ start, int dims,
-    int nseg, int zs, float inv, float *__restrict__ out, float scale_h, const float *__restrict__ scale_d, int fold)
+    const float4 *__restrict__ spos, const unsigned *__restrict__ start, int dims, int nseg, int zs, float inv,
+    float *__restrict__ out, float scale_h, const float *__restrict__ scale_d, int fold)
 {
     using SH = SdShape<MAS>;
     constexpr int S = SH::S, NT = SH::NT, H = S - 1, FL = SH::FL, PAD = SH::PAD, ZB = SH::ZB;
@@ -341,10 +370,9 @@ __global__ void __launch_bounds__(SDX * SDY, MAS == PYL_MAS_PCS ? 1 : 2) sd_depo
     auto first_from = [&](int z) {
         const unsigned *t = start + (long long)col * nseg + z / SD_Z;
         unsigned lo = t[0], hi = t[1];
-        const unsigned key = col * (unsigned)dims + (unsigned)z;
         while (lo < hi) {
             const unsigned mid = lo + (hi - lo) / 2;
-            if (keys[mid] < key) lo = mid + 1; else hi = mid;
+            if (sd_cell<MAS>(__ldg(spos + mid).z, inv, dims) < z) lo = mid + 1; else hi = mid;
         }
         return lo;
     };
@@ -363,7 +391,7 @@ __global__ void __launch_bounds__(SDX * SDY, MAS == PYL_MAS_PCS ? 1 : 2) sd_depo
     unsigned j = 0;
     float4 p = make_float4(0.0f, 0.0f, 0.0f, 0.0f), p2 = p;
     int layer = -1;
-    auto layer_of = [&]() { return j < col_end ? wrap_index(sd_first<MAS>(p.z, inv), dims) : -1; };
+    auto layer_of = [&]() { return j < col_end ? sd_cell<MAS>(p.z, inv, dims) : -1; };
     const int layers = z1 - z0 + H;
     for (int k0 = 0; k0 < layers; k0 += ZB) {                // base layers z0 - H + k0 ..
 #pragma unroll 1
@@ -447,25 +475,27 @@ __global__ void __launch_bounds__(SDX * SDY, MAS == PYL_MAS_PCS ? 1 : 2) sd_depo
 // NGP: a thread per cell finds its particles in the column's segment (cell = key) and
 // adds them in index order onto the grid's value (fold), as the serial loop does.
 template <bool WEIGHTED>
-__global__ void __launch_bounds__(256) sd_ngp_kernel(const float4 *__restrict__ spos, const unsigned *__restrict__ keys,
-                                                     const unsigned *__restrict__ start, int dims, int nseg,
-                                                     long long cells, float *__restrict__ out, float scale_h,
+__global__ void __launch_bounds__(256) sd_ngp_kernel(const float4 *__restrict__ spos, const unsigned *__restrict__ start,
+                                                     int dims, int nseg, float inv, long long cells,
+                                                     float *__restrict__ out, float scale_h,
                                                      const float *__restrict__ scale_d, int fold)
 {
     const long long stride = (long long)gridDim.x * blockDim.x;
     const float scale = scale_d ? *scale_d : scale_h;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < cells; i += stride) {
         const unsigned key = (unsigned)i;
-        const unsigned *t = start + (long long)(key / (unsigned)dims) * nseg + key % (unsigned)dims / SD_Z;
+        const int z = (int)(key % (unsigned)dims);
+        const unsigned *t = start + (long long)(key / (unsigned)dims) * nseg + z / SD_Z;
         unsigned lo = t[0], hi = t[1];
         const unsigned end = hi;
+        auto cell = [&](unsigned j) { return sd_cell<PYL_MAS_NGP>(__ldg(spos + j).z, inv, dims); };
         while (lo < hi) {
             const unsigned mid = lo + (hi - lo) / 2;
-            if (keys[mid] < key) lo = mid + 1; else hi = mid;
+            if (cell(mid) < z) lo = mid + 1; else hi = mid;
         }
-        if (lo >= end || keys[lo] != key) continue;
+        if (lo >= end || cell(lo) != z) continue;
         float v = fold ? out[i] : 0.0f;
-        for (; lo < end && keys[lo] == key; lo++) v = __fadd_rn(v, WEIGHTED ? __ldg(spos + lo).w : 1.0f);
+        for (; lo < end && cell(lo) == z; lo++) v = __fadd_rn(v, WEIGHTED ? __ldg(spos + lo).w : 1.0f);
         if (fold) out[i] = v;
         else if (v != 0.0f) out[i] = __fadd_rn(out[i], __fmul_rn(v, scale));
     }
@@ -474,9 +504,8 @@ __global__ void __launch_bounds__(256) sd_ngp_kernel(const float4 *__restrict__ 
 inline size_t al(size_t v) { return (v + 255) / 256 * 256; }
 
 struct SortedWs {
-    unsigned *k0, *v0, *k1, *v1, *hist, *partial;
-    unsigned *start;
-    float4 *spos;
+    float4 *rec[2];
+    unsigned *hist, *partial, *start;
     unsigned tiles;
     long long hist_len, parts, entries;      // entries: dims^2 * segments of a column
     size_t bytes;
@@ -491,14 +520,11 @@ SortedWs sorted_layout(void *base, long long n, int dims)
     w.parts = (w.hist_len + SCAN_BLOCK - 1) / SCAN_BLOCK;
     char *b = (char *)base;
     size_t o = 0;
-    w.k0 = (unsigned *)(b + o); o = al(o + 4 * (size_t)n);
-    w.v0 = (unsigned *)(b + o); o = al(o + 4 * (size_t)n);
-    w.k1 = (unsigned *)(b + o); o = al(o + 4 * (size_t)n);
-    w.v1 = (unsigned *)(b + o); o = al(o + 4 * (size_t)n);
+    w.rec[0] = (float4 *)(b + o); o = al(o + 16 * (size_t)n);
+    w.rec[1] = (float4 *)(b + o); o = al(o + 16 * (size_t)n);
     w.hist = (unsigned *)(b + o); o = al(o + 4 * (size_t)w.hist_len);
     w.partial = (unsigned *)(b + o); o = al(o + 4 * (size_t)w.parts);
     w.start = (unsigned *)(b + o); o = al(o + 4 * (size_t)(w.entries + 1));
-    w.spos = (float4 *)(b + o); o = al(o + 16 * (size_t)n);
     w.bytes = o;
     return w;
 }
@@ -510,45 +536,53 @@ inline unsigned blocks_for(long long n, int threads, int per_sm)
     return (unsigned)(b < 1 ? 1 : (b > cap ? cap : b));
 }
 
-// One grid: keys of the (shifted, for SHIFT) positions, stable radix sort, column starts,
-// positions gathered into sorted order, deposit.
-template <int MAS, bool SHIFT>
+// One pass of the sort: histogram, scan, scatter.
+template <int MAS, bool FIRST, bool SHIFT, bool WEIGHTED>
+int sort_pass(const RsSource &src, long long n, int shift, const SortedWs &ws, float4 *out, cudaStream_t st)
+{
+    rs_hist_kernel<MAS, FIRST, SHIFT, WEIGHTED><<<ws.tiles, RS_THREADS, 0, st>>>(src, n, shift, ws.tiles, ws.hist);
+    PYL_LAUNCH_CHECK();
+    scan_reduce_kernel<<<(unsigned)ws.parts, SCAN_THREADS, 0, st>>>(ws.hist, ws.hist_len, ws.partial);
+    PYL_LAUNCH_CHECK();
+    scan_partials_kernel<<<1, SCAN_THREADS, 0, st>>>(ws.partial, ws.parts);
+    PYL_LAUNCH_CHECK();
+    scan_apply_kernel<<<(unsigned)ws.parts, SCAN_THREADS, 0, st>>>(ws.hist, ws.hist_len, ws.partial);
+    PYL_LAUNCH_CHECK();
+    auto kern = rs_scatter_kernel<MAS, FIRST, SHIFT, WEIGHTED>;
+    PYL_CUDA(ensure_smem(kern, sizeof(RsSmem)));
+    kern<<<ws.tiles, RS_THREADS, sizeof(RsSmem), st>>>(src, n, shift, ws.tiles, ws.hist, out);
+    PYL_LAUNCH_CHECK();
+    return PYL_OK;
+}
+
+// One grid: stable radix sort of the (shifted, for SHIFT) particles by cell, column starts,
+// deposit.
+template <int MAS, bool SHIFT, bool WEIGHTED>
 int sorted_pass(const float *pos, const float *w, long long n, float *out, int dims, float inv, float halfcell,
                 const SortedWs &ws, float scale_h, const float *scale_d, bool fold, cudaStream_t st)
 {
     const long long cells = (long long)dims * dims * dims;
     stage_mark(PYL_STAGE_SORT, true, st);
-    sd_key_kernel<MAS, SHIFT><<<blocks_for(n, 256, 16), 256, 0, st>>>(pos, n, inv, halfcell, dims, ws.k0, ws.v0);
-    PYL_LAUNCH_CHECK();
     int bits = 1;
     while (bits < 32 && (1ull << bits) < (unsigned long long)cells) bits++;
-    unsigned *kin = ws.k0, *vin = ws.v0, *kout = ws.k1, *vout = ws.v1;
-    for (int shift = 0; shift < bits; shift += 8) {
-        rs_hist_kernel<<<ws.tiles, RS_THREADS, 0, st>>>(kin, n, shift, ws.tiles, ws.hist);
-        PYL_LAUNCH_CHECK();
-        scan_reduce_kernel<<<(unsigned)ws.parts, SCAN_THREADS, 0, st>>>(ws.hist, ws.hist_len, ws.partial);
-        PYL_LAUNCH_CHECK();
-        scan_partials_kernel<<<1, SCAN_THREADS, 0, st>>>(ws.partial, ws.parts);
-        PYL_LAUNCH_CHECK();
-        scan_apply_kernel<<<(unsigned)ws.parts, SCAN_THREADS, 0, st>>>(ws.hist, ws.hist_len, ws.partial);
-        PYL_LAUNCH_CHECK();
-        rs_scatter_kernel<<<ws.tiles, RS_THREADS, 0, st>>>(kin, vin, n, shift, ws.tiles, ws.hist, kout, vout);
-        PYL_LAUNCH_CHECK();
-        unsigned *t = kin; kin = kout; kout = t;
-        t = vin; vin = vout; vout = t;
+    RsSource src{pos, w, nullptr, inv, halfcell, dims};
+    for (int pass = 0; 8 * pass < bits; pass++) {
+        float4 *to = ws.rec[pass & 1];
+        const int rc = pass == 0 ? sort_pass<MAS, true, SHIFT, WEIGHTED>(src, n, 0, ws, to, st)
+                                 : sort_pass<MAS, false, false, WEIGHTED>(src, n, 8 * pass, ws, to, st);
+        if (rc) return rc;
+        src.rec = to;
     }
+    const float4 *spos = src.rec;
     const int nseg = (dims + SD_Z - 1) / SD_Z;
-    sd_start_kernel<<<blocks_for(n + 1, 256, 16), 256, 0, st>>>(kin, n, (unsigned)dims, (unsigned)nseg, ws.entries,
-                                                                ws.start);
-    PYL_LAUNCH_CHECK();
-    sd_gather_kernel<SHIFT><<<blocks_for(n, 256, 16), 256, 0, st>>>(pos, w, vin, n, halfcell, ws.spos);
+    sd_start_kernel<MAS, WEIGHTED><<<blocks_for(n + 1, 256, 16), 256, 0, st>>>(src, n, (unsigned)nseg, ws.entries, ws.start);
     PYL_LAUNCH_CHECK();
     stage_mark(PYL_STAGE_SORT, false, st);
     stage_mark(PYL_STAGE_DEPOSIT, true, st);
     const int f = fold ? 1 : 0;
     if constexpr (MAS == PYL_MAS_NGP) {
-        auto kern = w ? sd_ngp_kernel<true> : sd_ngp_kernel<false>;
-        kern<<<blocks_for(cells, 256, 32), 256, 0, st>>>(ws.spos, kin, ws.start, dims, nseg, cells, out, scale_h, scale_d, f);
+        sd_ngp_kernel<WEIGHTED><<<blocks_for(cells, 256, 32), 256, 0, st>>>(spos, ws.start, dims, nseg, inv, cells, out,
+                                                                            scale_h, scale_d, f);
     } else {
         constexpr int H = MAS - 1;
         // layers per CTA: SD_CTA_LAYERS, or fewer (each CTA brings its own S-1 halo layers)
@@ -557,10 +591,10 @@ int sorted_pass(const float *pos, const float *w, long long n, float *out, int d
         int zs = SD_CTA_LAYERS;
         while (zs > 8 && (long long)gx * gy * ((dims + zs - 1) / zs) < 2LL * num_sms()) zs /= 2;
         constexpr size_t smem = SdShape<MAS>::SMEM;
-        auto kern = w ? sd_deposit_kernel<MAS, true> : sd_deposit_kernel<MAS, false>;
+        auto kern = sd_deposit_kernel<MAS, WEIGHTED>;
         PYL_CUDA(ensure_smem(kern, smem));
         kern<<<dim3((unsigned)((dims + zs - 1) / zs), gy, gx), dim3(SDY, SDX), smem, st>>>(
-            ws.spos, kin, ws.start, dims, nseg, zs, inv, out, scale_h, scale_d, f);
+            spos, ws.start, dims, nseg, zs, inv, out, scale_h, scale_d, f);
     }
     PYL_LAUNCH_CHECK();
     stage_mark(PYL_STAGE_DEPOSIT, false, st);
@@ -572,9 +606,11 @@ int sorted_run(const float *pos, const float *w, long long n, float *grid, float
                float halfcell, void *workspace, float scale_h, const float *scale_d, bool fold, cudaStream_t st)
 {
     const SortedWs ws = sorted_layout(workspace, n, dims);
-    int rc = sorted_pass<MAS, false>(pos, w, n, grid, dims, inv, halfcell, ws, scale_h, scale_d, fold, st);
+    auto plain = w ? sorted_pass<MAS, false, true> : sorted_pass<MAS, false, false>;
+    auto shifted = w ? sorted_pass<MAS, true, true> : sorted_pass<MAS, true, false>;
+    const int rc = plain(pos, w, n, grid, dims, inv, halfcell, ws, scale_h, scale_d, fold, st);
     if (rc || !grid2) return rc;
-    return sorted_pass<MAS, true>(pos, w, n, grid2, dims, inv, halfcell, ws, scale_h, scale_d, fold, st);
+    return shifted(pos, w, n, grid2, dims, inv, halfcell, ws, scale_h, scale_d, fold, st);
 }
 
 }  // namespace
