@@ -165,12 +165,13 @@ int pyl_scale(float *p, int64_t n, float factor, void *stream);
 /* Batched realizations through the tiled binning (no counterpart in the
  * reference): every realization's grid is cut into 32^3-cell bins numbered
  * tile_base[r] + (tx*nt + ty)*nt + tz (nt = ceil(dims/32), dims <= 512;
- * realizations with larger grids are skipped), total_tiles bins in all.  Four
- * stream-ordered launches: per-item bin histograms, a scan, per-item placement,
- * and one persistent deposit over all bins (10.22 fixed point per bin, the
+ * realizations with larger grids are skipped), total_tiles bins in all.
+ * Stream-ordered launches: per-item bin histograms, a scan, per-item placement, a
+ * list of the bins or parts of crowded bins, and one persistent deposit over it (10.22 fixed point per bin, the
  * realization's MAS and interlacing), adding scale * deposit into the grids
  * (pre-filled by the caller, e.g. with -1 for the overdensity).  reals, items
- * and tile_base live in device memory; total_particles = sum of item counts. */
+ * and tile_base live in device memory; total_particles = sum of item counts.
+ * ctas_per_sm (1..8) is checked; every launch here has its own grid. */
 size_t pyl_ma_batch_tiled_workspace_size(uint32_t total_tiles, int64_t total_particles);
 int pyl_ma_batch_tiled(const pyl_batch_real *reals, int n_reals, const pyl_batch_item *items, int n_items,
                        const uint32_t *tile_base, uint32_t total_tiles, int64_t total_particles, void *workspace,

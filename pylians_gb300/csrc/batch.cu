@@ -108,7 +108,13 @@ __global__ void __launch_bounds__(256) scale_value_kernel(float *g, long long n,
 //               24 realizations up to 256^3: 3.0 ms with whole bins (2.3 ms of it
 //               one bin of a 64^3 grid), 1.9 ms in parts.
 constexpr int BT_MAX_TILES = 4096;        // bins per realization (dims <= 512)
-constexpr int BT_BATCH = 4096;            // placement batch (particles)
+// Count and placement: threads per CTA, CTAs per SM.  One CTA of 1024 threads (its 50
+// registers leave no room for a second) stood still at every barrier and reservation: 24
+// realizations of 70 million particles 823 us for the placement, 236 for the count; three
+// of 512 threads 733 and 202 (five of 256: 826 and 242).  The placement is bound by the
+// random shared-memory accesses of its sort (60 % of the wavefronts) and by barriers.
+constexpr int BT_THREADS = 512, BT_CTAS = 3;
+constexpr int BT_BATCH = 4 * BT_THREADS;     // placement batch (particles)
 
 __device__ __forceinline__ int bt_nt(int dims) { return (dims + TB - 1) / TB; }
 
@@ -154,7 +160,7 @@ __device__ __forceinline__ void load_quad(const float *pos, long long q, long lo
     }
 }
 
-__global__ void __launch_bounds__(1024) bt_count_kernel(const pyl_batch_real *__restrict__ reals,
+__global__ void __launch_bounds__(BT_THREADS, BT_CTAS) bt_count_kernel(const pyl_batch_real *__restrict__ reals,
                                                         const pyl_batch_item *__restrict__ items, int n_items,
                                                         const unsigned *__restrict__ tile_base,
                                                         unsigned *__restrict__ counts, unsigned *counter)
@@ -337,17 +343,14 @@ __global__ void __launch_bounds__(1024) bt_scan_kernel(const unsigned *__restric
     if (threadIdx.x == blockDim.x - 1) offsets[n] = (unsigned)part[threadIdx.x];
 }
 
-// Exclusive scan of v[0..n) in place, n <= 4 * blockDim.x (each thread four
-// consecutive entries); warp_tot: 32 entries of scratch.  All threads call it.
-__device__ __forceinline__ void bt_block_scan4(unsigned *v, int n, unsigned *warp_tot)
+// Exclusive scan of v[0..n) in place (each thread n / blockDim.x consecutive entries);
+// warp_tot: 32 entries of scratch.  All threads call it.
+__device__ __forceinline__ void bt_block_scan(unsigned *v, int n, unsigned *warp_tot)
 {
     const int t = threadIdx.x, lane = t & 31, w = t >> 5, nw = (blockDim.x + 31) >> 5;
-    unsigned x[4], tot = 0;
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-        x[k] = 4 * t + k < n ? v[4 * t + k] : 0u;
-        tot += x[k];
-    }
+    const int per = (n + blockDim.x - 1) / blockDim.x, first = per * t, last = min(n, first + per);
+    unsigned tot = 0;
+    for (int i = first; i < last; i++) tot += v[i];
     unsigned inc = tot;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -368,23 +371,22 @@ __device__ __forceinline__ void bt_block_scan4(unsigned *v, int n, unsigned *war
     }
     __syncthreads();
     unsigned run = inc - tot + warp_tot[w];
-#pragma unroll
-    for (int k = 0; k < 4; k++)
-        if (4 * t + k < n) {
-            v[4 * t + k] = run;
-            run += x[k];
-        }
+    for (int i = first; i < last; i++) {
+        const unsigned x = v[i];
+        v[i] = run;
+        run += x;
+    }
     __syncthreads();
 }
 
-// Per 4096-particle batch of an item: ranks per bin from shared-memory counters,
+// Per BT_BATCH particles of an item: ranks per bin from shared-memory counters,
 // one global atomic per bin touched reserves its run in the bin's range, the batch
 // is sorted by bin in shared memory, and the runs are written out coalesced
 // (consecutive threads, consecutive slots of a run).
 constexpr size_t BT_PLACE_SMEM = sizeof(unsigned) * 2 * BT_MAX_TILES + sizeof(float4) * BT_BATCH +
                                  sizeof(unsigned short) * BT_BATCH;
 
-__global__ void __launch_bounds__(1024) bt_place_kernel(const pyl_batch_real *__restrict__ reals,
+__global__ void __launch_bounds__(BT_THREADS, BT_CTAS) bt_place_kernel(const pyl_batch_real *__restrict__ reals,
                                                         const pyl_batch_item *__restrict__ items, int n_items,
                                                         const unsigned *__restrict__ tile_base,
                                                         unsigned *__restrict__ cursor, unsigned n_total,
@@ -396,7 +398,7 @@ __global__ void __launch_bounds__(1024) bt_place_kernel(const pyl_batch_real *__
     unsigned short *skey = (unsigned short *)(stage + BT_BATCH);
     __shared__ unsigned wt[32];
     __shared__ int cur;
-    constexpr int U = BT_BATCH / 1024;
+    constexpr int U = BT_BATCH / BT_THREADS;
     static_assert(U == 4, "four particles per thread and batch");
     static_assert(BT_MAX_TILES <= 65536, "bin keys held as 16 bits");
     for (;;) {
@@ -421,7 +423,7 @@ __global__ void __launch_bounds__(1024) bt_place_kernel(const pyl_batch_real *__
             float4 v[U];
             int key[U];
             unsigned rank[U];
-            // thread t takes particles s0 + 4t .. s0 + 4t + 3 (BT_BATCH = 4 x 1024)
+            // thread t takes particles s0 + 4t .. s0 + 4t + 3 (BT_BATCH = 4 BT_THREADS)
             float p[U][3];
             load_quad(r.pos, s0 + 4 * threadIdx.x, end, vec, p);
 #pragma unroll
@@ -438,7 +440,7 @@ __global__ void __launch_bounds__(1024) bt_place_kernel(const pyl_batch_real *__
             for (int t = threadIdx.x; t < ntiles; t += blockDim.x)
                 if (bcnt[t]) gbase[t] = atomicAdd(cursor + base + t, bcnt[t]);
             __syncthreads();
-            bt_block_scan4(bcnt, ntiles, wt);                  // bcnt: the batch's run starts
+            bt_block_scan(bcnt, ntiles, wt);                   // bcnt: the batch's run starts
 #pragma unroll
             for (int u = 0; u < U; u++)
                 if (key[u] >= 0) {
@@ -699,13 +701,13 @@ extern "C" int pyl_ma_batch_tiled(const pyl_batch_real *reals, int n_reals, cons
     PYL_CUDA(cudaMemsetAsync(ws.counts, 0, 4 * ((size_t)total_tiles + 1), st));
     PYL_CUDA(cudaMemsetAsync(ws.counters, 0, ws.zero_bytes, st));
     if (n_items == 0) return PYL_OK;
-    const unsigned grid = (unsigned)(num_sms() * ctas_per_sm);
-    bt_count_kernel<<<grid, 1024, 0, st>>>(reals, items, n_items, tile_base, ws.counts, ws.counters);
+    const unsigned grid = (unsigned)(num_sms() * BT_CTAS);
+    bt_count_kernel<<<grid, BT_THREADS, 0, st>>>(reals, items, n_items, tile_base, ws.counts, ws.counters);
     PYL_LAUNCH_CHECK();
     bt_scan_kernel<<<1, 1024, 0, st>>>(ws.counts, total_tiles, ws.offsets, ws.cursor);
     PYL_LAUNCH_CHECK();
     PYL_CUDA(ensure_smem(bt_place_kernel, BT_PLACE_SMEM));
-    bt_place_kernel<<<grid, 1024, BT_PLACE_SMEM, st>>>(reals, items, n_items, tile_base, ws.cursor,
+    bt_place_kernel<<<grid, BT_THREADS, BT_PLACE_SMEM, st>>>(reals, items, n_items, tile_base, ws.cursor,
                                                        (unsigned)total_particles, ws.rec, ws.counters + 1);
     PYL_LAUNCH_CHECK();
     const unsigned max_parts = (unsigned)bt_max_parts(total_tiles), sms = (unsigned)num_sms();
