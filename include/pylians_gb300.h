@@ -38,12 +38,13 @@ extern "C" {
 #define PYL_MAS_PCS 4
 
 /* scatter strategies for pyl_ma */
-#define PYL_STRATEGY_AUTO 0   /* library picks by grid size and particle count */
+#define PYL_STRATEGY_AUTO 0   /* library picks by grid size and particle count (unweighted NGP on
+                                 grids in L2: whole-number counts, when the workspace holds them) */
 #define PYL_STRATEGY_ATOMIC 1 /* one thread per particle, atomics into the grid */
 #define PYL_STRATEGY_TILED 2  /* bin particles by tile, deposit tiles in shared memory;
                                  3D; calls of 2^32 - 4096 particles and more run as
                                  consecutive passes (pyl_ma_set_pass_limit) */
-#define PYL_STRATEGY_SORTED 3 /* radix sort by cell + fixed-order per-cell gather: bit-reproducible */
+#define PYL_STRATEGY_SORTED 3 /* radix sort by cell + fixed-order column sums: bit-reproducible */
 
 const char *pyl_strerror(int status);
 /* Detail of the last failure on the calling host thread ("" if none). */

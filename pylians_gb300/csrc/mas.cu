@@ -27,6 +27,7 @@
 
 #include <stdlib.h>
 
+#include <algorithm>
 #include <atomic>
 #include <map>
 #include <mutex>
@@ -149,6 +150,83 @@ int launch_atomic(const float *pos, const float *w, long long n, float *grid, fl
     return PYL_OK;
 }
 
+// ------------------------------------------------------------------ NGP counts
+// Unweighted NGP on grids that stay in L2: whole-number counts by red.global, a run of
+// lanes in one cell as one addition, then one pass adds them to the grids: the bits of the
+// tiled deposit, which rounds a cell's total once too.  Bound by the additions in L2; with
+// one addition a particle the tiled deposit's passes (count, placement, deposit) cost more.
+// Particles in no order, counts and tiled (us):
+//   256^3 particles: 64^3 122 and 855, 128^3 126 and 337, 256^3 184 and 318; interlaced
+//   200^3 234 and 474;  400^3 on 128^3 373 and 1121;  2^20 on 256^3 83 and 84.
+// Past NGP_COUNT_BYTES the counts leave L2 (256^3 interlaced, 128 MB: 587 us without their
+// passes, 466 tiled), and past NGP_COUNT_PER_CELL the additions to one cell queue (400^3 on 16^3:
+// 1470 and 1353).
+template <bool INTERLACED>
+__global__ void __launch_bounds__(256) ngp_count_kernel(const float *__restrict__ pos, long long n, int dims, float inv,
+                                                        float halfcell, unsigned *__restrict__ cnt,
+                                                        unsigned *__restrict__ cnt2)
+{
+    const int lane = threadIdx.x & 31;
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const bool valid = i < n;
+    float p[3] = {0.0f, 0.0f, 0.0f};
+    if (valid)
+#pragma unroll
+        for (int a = 0; a < 3; a++) p[a] = __ldg(pos + 3 * i + a);
+#pragma unroll
+    for (int g = 0; g < (INTERLACED ? 2 : 1); g++) {
+        unsigned cell = 0;
+#pragma unroll
+        for (int a = 0; a < 3; a++) {
+            const float q = g == 0 ? p[a] : __fadd_rn(p[a], halfcell);
+            cell = cell * (unsigned)dims + (unsigned)wrap_index(axis_first<PYL_MAS_NGP>(q, inv), dims);
+        }
+        if (!valid) cell = 0xffffffffu;
+        const unsigned prev = __shfl_up_sync(0xffffffffu, cell, 1);
+        const bool head = lane == 0 || cell != prev;
+        const unsigned heads = __ballot_sync(0xffffffffu, head), after = heads & ~((2u << lane) - 1u);
+        if (head && valid) atomicAdd((g == 0 ? cnt : cnt2) + cell, (unsigned)((after ? __ffs(after) - 1 : 32) - lane));
+    }
+}
+
+__global__ void __launch_bounds__(256) ngp_add_kernel(const unsigned *__restrict__ cnt, long long cells,
+                                                      float *__restrict__ grid, float *__restrict__ grid2)
+{
+    const long long stride = (long long)gridDim.x * blockDim.x, total = grid2 ? 2 * cells : cells;
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
+        const unsigned c = cnt[i];
+        float *g = i < cells ? grid + i : grid2 + (i - cells);
+        if (c) *g = __fadd_rn(*g, (float)c);
+    }
+}
+
+constexpr long long NGP_COUNT_BYTES = 64ll << 20, NGP_COUNT_PER_CELL = 4096;
+
+// Bytes of the counts of an unweighted NGP deposit that takes them, 0 for the others.
+inline size_t ngp_count_bytes(int mas, int strategy, int ndim, int dims, long long n, bool inter)
+{
+    const long long bytes = 4ll * dims * dims * dims * (inter ? 2 : 1);
+    const bool counts = mas == PYL_MAS_NGP && strategy == PYL_STRATEGY_AUTO && ndim == 3 && dims <= 256 &&
+                        bytes <= NGP_COUNT_BYTES && n >= (1ll << 20) && n < 0xFFFFFFFFll &&
+                        n <= NGP_COUNT_PER_CELL * dims * dims * dims;
+    return counts ? (size_t)bytes : 0;
+}
+
+int launch_ngp_counts(const float *pos, long long n, float *grid, float *grid2, int dims, float inv, float halfcell,
+                      void *workspace, cudaStream_t st)
+{
+    const long long cells = (long long)dims * dims * dims;
+    unsigned *cnt = (unsigned *)workspace;
+    PYL_CUDA(cudaMemsetAsync(cnt, 0, 4 * (size_t)cells * (grid2 ? 2 : 1), st));
+    const unsigned blocks = (unsigned)((n + 255) / 256);
+    if (grid2) ngp_count_kernel<true><<<blocks, 256, 0, st>>>(pos, n, dims, inv, halfcell, cnt, cnt + cells);
+    else       ngp_count_kernel<false><<<blocks, 256, 0, st>>>(pos, n, dims, inv, halfcell, cnt, nullptr);
+    PYL_LAUNCH_CHECK();
+    ngp_add_kernel<<<grid_blocks(cells, 256, 16), 256, 0, st>>>(cnt, cells, grid, grid2);
+    PYL_LAUNCH_CHECK();
+    return PYL_OK;
+}
+
 // AUTO: binning pays once a deposit has about a million particles and several per
 // bin; below that, red.global into an L2-resident grid wins.
 inline int pick_strategy(int strategy, int ndim, int dims, long long n)
@@ -172,10 +250,12 @@ extern "C" size_t pyl_ma_workspace_size(int64_t n_particles, int ndim, int dims,
     // + 256 bytes at the end: the mass sum and scale of pyl_ma_overdensity
     if (s == PYL_STRATEGY_SORTED && ndim == 3 && sorted_supported(n_particles, dims))
         return sorted_workspace_bytes(n_particles, dims) + 256;
+    size_t bytes = ngp_count_bytes(mas, strategy, ndim, dims, n_particles, interlaced != 0);
     if (s == PYL_STRATEGY_TILED && ndim == 3)
-        return tiled_layout(nullptr, tiled_pass_len(n_particles), dims,
-                            tiled_extra_bytes(tiled_pass_len(n_particles), mas, dims, interlaced != 0)).bytes + 256;
-    return 256;
+        bytes = std::max(bytes, tiled_layout(nullptr, tiled_pass_len(n_particles), dims,
+                                             tiled_extra_bytes(tiled_pass_len(n_particles), mas, dims, interlaced != 0))
+                                    .bytes);
+    return bytes + 256;
 }
 
 extern "C" int pyl_ma(const float *pos, const float *weights, int64_t n, int ndim, float *grid,
@@ -214,6 +294,9 @@ extern "C" int pyl_ma(const float *pos, const float *weights, int64_t n, int ndi
                              nullptr, true, st);
     }
     if (s == PYL_STRATEGY_TILED && ndim != 3) s = PYL_STRATEGY_ATOMIC;
+    const size_t counts = weights ? 0 : ngp_count_bytes(mas, strategy, ndim, dims, n, grid_interlaced != nullptr);
+    if (counts && workspace != nullptr && workspace_bytes >= counts && ((uintptr_t)workspace & 3) == 0)
+        return launch_ngp_counts(pos, n, grid, grid_interlaced, dims, inv, halfcell, workspace, st);
     Owned ow{false, nullptr, 0, 0.0f, 0, false};
     const long long pass = tiled_pass_len(n);
     if (s == PYL_STRATEGY_TILED) {
