@@ -1,7 +1,7 @@
 // Spectra from the float64 sums of pyl_pk_bin, on the host: Pk_library.pyx:384-421 (Pk) and
 // :740-796 (XPk).  One pass over the bins writes every result array, in the order of
 // operations of those lines.  As numpy expressions (a temporary for each operation, a
-// scatter for kpar and kper) four fields of 128^3 took 0.25 ms, one of 1024^3 7.0 ms for
+// scatter for kpar and kper) four fields of 128^3 took 0.25 ms, two of 1023^3 7.0 ms for
 // 0.08 and 1.2 ms here; Pk of 128^3 0.29 -> 0.20 ms, XPk of two 512^3 5.44 -> 4.05 ms.
 // Bound by the pages of the results (372,000 k_par/k_per bins at 1024^3) and the divisions.
 #include <cmath>
