@@ -52,162 +52,24 @@ __global__ void __launch_bounds__(512) xi_power_kernel(float2 *dk, PkDims d, int
     }
 }
 
-// sums: X[nb3][3] | R[nb3] | N[nb3] (float64).
+// sums: X[nb3][3] | R[nb3] | N[nb3] (float64)
 //
-// |r|, its bin and every Legendre weight are the same for the eight separations
-// (+-rx, +-ry, +-rz): a warp adds the (up to eight) values per rz from coalesced reads
-// of the four sign rows and their mirrored halves into shared memory, and each lane
-// walks its run of rz (an odd number of them: distinct banks), adding to the CTA's
-// shared sums only when the bin changes (bins below `core`: counts and R alone,
-// xi_row_kernel has their values).  One thread per row, 4 bytes at a time and
-// 1 KB apart, took 0.62 ms for 256^3, and float64 roots of every separation for R
-// another 1.45 ms; this kernel takes 0.05 ms (0.30 ms for 512^3).  Counts are exact in float32: the CTAs
-// share a bin's 4 pi r^2 separations, far below 2^24 each.  R adds |r| in float64 over
-// ry >= rx only, twice off the diagonal.
-struct XiRun {
-    int segments, run;
-};
-
-inline XiRun xi_run(int nz)
-{
-    XiRun x;
-    x.segments = (nz + 32 * 9 - 1) / (32 * 9);
-    x.run = ((nz + 32 * x.segments - 1) / (32 * x.segments)) | 1;
-    return x;
-}
-
-constexpr int XI_WARPS = 8;
-constexpr int XI_CORE = 32;              // bins that xi_row_kernel sums on large grids
-constexpr int XI_ROWS_BELOW = 256;       // grids whose every bin it sums
-
-inline size_t xi_smem(const PkDims &d, const XiRun &x)
-{
-    return (size_t)d.nb3 * (sizeof(double) + 4 * sizeof(float)) + sizeof(float) * XI_WARPS * 32 * x.run;
-}
-
-// |r| to float64 from the float32 square root and one Newton correction: relative
-// error below 2^-47 of each term (n2 < 2^24 is exact in float32).
-__device__ __forceinline__ double length_of(int n2)
-{
-    if (n2 == 0) return 0.0;
-    const float f = (float)n2, s = sqrtf(f);
-    const float e = __fmaf_rn(-s, s, f);                 // exact residual
-    return (double)s + (double)__fdividef(e, 2.0f * s);
-}
-
-__global__ void __launch_bounds__(32 * XI_WARPS) xi_bin_kernel(const float *__restrict__ xi, PkDims d, int axis,
-                                                               XiRun x, int core, double *__restrict__ sums)
-{
-    extern __shared__ __align__(16) double xsm[];
-    const int dims = d.dims, nb = d.nb3;
-    double *R = xsm;
-    float *acc = (float *)(xsm + nb);                    // [nb3][4]: l = 0, 2, 4, count
-    float *stage = acc + 4 * nb + (threadIdx.x >> 5) * 32 * x.run;
-    for (int i = threadIdx.x; i < nb; i += blockDim.x) {
-        R[i] = 0.0;
-        acc[4 * i] = acc[4 * i + 1] = acc[4 * i + 2] = acc[4 * i + 3] = 0.0f;
-    }
-    __syncthreads();
-    const int G = sym_groups(dims), lane = threadIdx.x & 31;
-    const int nwarp = (int)(gridDim.x * XI_WARPS), slots = 32 * x.run;
-    for (int rep = (int)(blockIdx.x * XI_WARPS + (threadIdx.x >> 5)); rep < G * G; rep += nwarp) {
-        const int xr = rep / G, yr = rep % G;
-        const int nx = (xr == 0 || 2 * xr == dims) ? 1 : 2, ny = (yr == 0 || 2 * yr == dims) ? 1 : 2;
-        const int rows = nx * ny, rho2 = xr * xr + yr * yr;
-        long long off[4];
-#pragma unroll
-        for (int r = 0; r < 4; r++) {
-            const int ix = ((r & 1) && nx == 2) ? dims - xr : xr, iy = ((r & 2) && ny == 2) ? dims - yr : yr;
-            off[r] = ((long long)ix * dims + iy) * dims;
-        }
-        const unsigned used = 1u | (nx == 2 ? 2u : 0u) | (ny == 2 ? 4u : 0u) | (rows == 4 ? 8u : 0u);
-        for (int sgm = 0; sgm < x.segments; sgm++) {
-            const int k0 = sgm * slots, k1 = min(d.nz, k0 + slots);
-            for (int z = k0 + lane; core < nb && z < k1; z += 32) {
-                const bool two = z != 0 && 2 * z != dims;
-                float a[4], b[4];
-#pragma unroll
-                for (int r = 0; r < 4; r++) {
-                    a[r] = (used >> r) & 1u ? __ldg(xi + off[r] + z) : 0.0f;
-                    b[r] = two && ((used >> r) & 1u) ? __ldg(xi + off[r] + dims - z) : 0.0f;
-                }
-                stage[z - k0] = ((a[0] + b[0]) + (a[1] + b[1])) + ((a[2] + b[2]) + (a[3] + b[3]));
-            }
-            __syncwarp();
-            const int kb = k0 + lane * x.run, ke = min(k1, kb + x.run);
-            if (kb < ke) {
-                int n2 = rho2 + kb * kb;
-                int bin = isqrt_exact(n2);
-                float s0 = 0.0f, s2 = 0.0f, s4 = 0.0f, c = 0.0f;
-                double len = 0.0;
-                const int par2 = axis == 0 ? xr * xr : yr * yr;
-                const float wl = yr > xr ? 2.0f : 1.0f;
-                for (int z = kb; z < ke; z++) {
-                    // correctly rounded, as the float64 quotient rounded to float32 is
-                    // (both operands are integers below 2^24)
-                    const float mu2 = n2 ? __fdiv_rn((float)(axis == 2 ? z * z : par2), (float)n2) : 0.0f;
-                    const float v = stage[z - k0];
-                    const float m = (float)(rows * (z != 0 && 2 * z != dims ? 2 : 1));
-                    if (bin >= core) {
-                        s0 += v;
-                        s2 += v * (0.5f * (3.0f * mu2 - 1.0f));
-                        s4 += v * (0.125f * ((35.0f * mu2 - 30.0f) * mu2 + 3.0f));
-                    }
-                    c += m;
-                    if (yr >= xr) len += (double)(wl * m) * length_of(n2);
-                    n2 += 2 * z + 1;
-                    const bool next = (bin + 1) * (bin + 1) <= n2;
-                    if (next || z + 1 == ke) {
-                        atomicAdd(acc + 4 * bin, s0);
-                        atomicAdd(acc + 4 * bin + 1, s2);
-                        atomicAdd(acc + 4 * bin + 2, s4);
-                        atomicAdd(acc + 4 * bin + 3, c);
-                        if (len != 0.0) atomicAdd(R + bin, len);
-                        s0 = s2 = s4 = c = 0.0f;
-                        len = 0.0;
-                        bin += next ? 1 : 0;
-                    }
-                }
-            }
-            __syncwarp();
-        }
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < nb; i += blockDim.x) {
-        if (acc[4 * i + 3] == 0.0f) continue;
-#pragma unroll
-        for (int l = 0; l < 3; l++) atomicAdd(sums + 3 * i + l, (double)acc[4 * i + l]);
-        if (R[i] != 0.0) atomicAdd(sums + 3 * nb + i, R[i]);
-        atomicAdd(sums + 4 * nb + i, (double)acc[4 * i + 3]);
-    }
-}
-
-// The sums of the bins below `core`: XI_CORE of them, or every bin of grids below
-// XI_ROWS_BELOW, where they hold few separations each.  There the order of the float32
-// additions shows in xi (1e-8 of the largest multipole; the larger bins of larger grids
-// average it away), and the sums keep one order: a thread walks a row (rx, ry) along rz
-// in step with the other rows of its CTA and adds to the CTA's sums when its bin
-// changes.  Bound by the latency of a step, about 1.5 us: 0.09 ms for |rz| < XI_CORE of
-// the CTAs with rows of the core at 256^3; below that size whole rows take less than
-// 0.6 ms (0.53 ms at 200^3, where xi_bin_kernel would add the values in 0.03 ms).
-__global__ void __launch_bounds__(256) xi_row_kernel(const float *__restrict__ xi, PkDims d, int axis, int core,
+// A thread walks a row (rx, ry) along rz and adds to its CTA's float32 sums when the bin
+// changes; the CTAs' sums meet in float64.  The order and the widths of these additions
+// are part of the result: bins of few separations (the smallest and, in the corners of the
+// cube, the largest |r|) show them.  Adding the eight separations (+-rx, +-ry, +-rz) in
+// float32 first, in a kernel that took 0.05 ms for the 0.62 of this one at 256^3, lost the
+// smaller ones of different x planes, which meet in float64 here, and moved xi of 512^3 by
+// 1e-9 where two runs of this order differ by 2e-10.  Bound by the float32 shared-memory
+// additions (compare and swap): rows staged through shared memory took no less.
+__global__ void __launch_bounds__(256) xi_bin_kernel(const float *__restrict__ xi, PkDims d, int axis,
                                                      double *__restrict__ sums)
 {
-    extern __shared__ float acc[];                      // [nb3][3]; bins from `core` up are scratch
+    extern __shared__ float acc[];                      // [nb3][3]
     const int dims = d.dims, nb = d.nb3;
-    const long long rows = (long long)dims * dims;
-    bool any = false;
-    for (long long row = (long long)blockIdx.x * blockDim.x + threadIdx.x; row < rows;
-         row += (long long)gridDim.x * blockDim.x) {
-        const int rx = freq_of((int)(row / dims), dims), ry = freq_of((int)(row % dims), dims);
-        any |= rx * rx + ry * ry < core * core;
-    }
-    if (!__syncthreads_or(any)) return;
     for (int i = threadIdx.x; i < 3 * nb; i += blockDim.x) acc[i] = 0.0f;
     __syncthreads();
-    // rz = 0 .. up, then -down .. -1; with larger bins between them, a new run
-    const int up = min(core - 1, dims / 2), down = min(core - 1, (dims - 1) / 2);
-    const bool gap = up + 1 < dims - down;
+    const long long rows = (long long)dims * dims;
     for (long long row = (long long)blockIdx.x * blockDim.x + threadIdx.x; row < rows;
          row += (long long)gridDim.x * blockDim.x) {
         const int rx = freq_of((int)(row / dims), dims), ry = freq_of((int)(row % dims), dims);
@@ -215,14 +77,13 @@ __global__ void __launch_bounds__(256) xi_row_kernel(const float *__restrict__ x
         int cur = -1;
         float s0 = 0.0f, s2 = 0.0f, s4 = 0.0f;
         for (int zz = 0; zz < dims; zz++) {
-            if (gap && zz == up + 1) zz = dims - down;
             const int rz = freq_of(zz, dims);
             const int n2 = rx * rx + ry * ry + rz * rz;
             const int bin = isqrt_exact(n2);
             const int par = axis == 0 ? rx : (axis == 1 ? ry : rz);
             const float mu2 = n2 ? (float)((double)(par * par) / (double)n2) : 0.0f;
             const float v = __ldg(g + zz);
-            if (bin != cur || (gap && zz == dims - down)) {
+            if (bin != cur) {
                 if (cur >= 0) {
                     atomicAdd(acc + 3 * cur, s0);
                     atomicAdd(acc + 3 * cur + 1, s2);
@@ -242,8 +103,60 @@ __global__ void __launch_bounds__(256) xi_row_kernel(const float *__restrict__ x
         }
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < 3 * min(core, nb); i += blockDim.x)
+    for (int i = threadIdx.x; i < 3 * nb; i += blockDim.x)
         if (acc[i] != 0.0f) atomicAdd(sums + i, (double)acc[i]);
+}
+
+
+// Data-independent sums: R[bin] = sum |r|, N[bin] = count, over all dims^3 separations.
+// |r| and its bin are the same for (+-rx, +-ry, +-rz) and for rx and ry exchanged: a warp
+// takes a representative (|rx|, |ry|) with ry >= rx, its lanes a run of rz each, one
+// float64 root for up to sixteen separations.  A root for each separation took 1.45 ms at
+// 256^3, this 0.04 ms (512^3: 0.24 ms).
+constexpr int XI_WARPS = 8;
+__global__ void __launch_bounds__(32 * XI_WARPS) xi_geometry_kernel(PkDims d, double *__restrict__ sums)
+{
+    extern __shared__ __align__(16) double xsm[];
+    const int dims = d.dims, nb = d.nb3;
+    double *R = xsm;
+    unsigned *N = (unsigned *)(xsm + nb);
+    for (int i = threadIdx.x; i < nb; i += blockDim.x) {
+        R[i] = 0.0;
+        N[i] = 0u;
+    }
+    __syncthreads();
+    const int G = sym_groups(dims), lane = threadIdx.x & 31, run = (d.nz + 31) / 32;
+    const int nwarp = (int)(gridDim.x * XI_WARPS);
+    for (int rep = (int)(blockIdx.x * XI_WARPS + (threadIdx.x >> 5)); rep < G * G; rep += nwarp) {
+        const int xr = rep / G, yr = rep % G;
+        if (yr < xr) continue;
+        const int rows = ((xr == 0 || 2 * xr == dims) ? 1 : 2) * ((yr == 0 || 2 * yr == dims) ? 1 : 2) * (yr > xr ? 2 : 1);
+        const int kb = lane * run, ke = min(d.nz, kb + run);
+        if (kb >= ke) continue;
+        int n2 = xr * xr + yr * yr + kb * kb, bin = isqrt_exact(n2);
+        unsigned c = 0;
+        double len = 0.0;
+        for (int z = kb; z < ke; z++) {
+            const unsigned m = (unsigned)(rows * (z != 0 && 2 * z != dims ? 2 : 1));
+            c += m;
+            len += (double)m * sqrt((double)n2);
+            n2 += 2 * z + 1;
+            const bool next = (bin + 1) * (bin + 1) <= n2;
+            if (next || z + 1 == ke) {
+                atomicAdd(N + bin, c);
+                atomicAdd(R + bin, len);
+                c = 0u;
+                len = 0.0;
+                bin += next ? 1 : 0;
+            }
+        }
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < nb; i += blockDim.x) {
+        if (N[i] == 0u) continue;
+        atomicAdd(sums + 3 * nb + i, R[i]);
+        atomicAdd(sums + 4 * nb + i, (double)N[i]);
+    }
 }
 
 // correct_MAS's mode loop (Pk_library.pyx:1776-1794): every stored mode but the
@@ -354,18 +267,14 @@ extern "C" int pyl_xi_bin(const float *xi_grid, int dims, int axis, double *sums
     const PkDims d = pk_dims(dims);
     cudaStream_t st = (cudaStream_t)stream;
     PYL_CUDA(cudaMemsetAsync(sums, 0, sizeof(double) * 5 * d.nb3, st));
-    PYL_CHECK_ARG(sizeof(float) * 3 * d.nb3 <= 48 * 1024, "grid too large for the shared-memory bins");
-    const XiRun x = xi_run(d.nz);
-    const size_t smem = xi_smem(d, x);
-    PYL_CUDA(ensure_smem(xi_bin_kernel, smem));
-    // one wave of resident CTAs, at least two representatives a warp
-    const long long reps = (long long)sym_groups(dims) * sym_groups(dims);
-    const long long per_sm = std::max<long long>(1, std::min<long long>(6, (long long)(227 * 1024 / (smem + 1024))));
-    const long long b = std::min((reps + 2 * XI_WARPS - 1) / (2 * XI_WARPS), per_sm * num_sms());
-    const int core = dims < XI_ROWS_BELOW ? d.nb3 : XI_CORE;
-    xi_bin_kernel<<<(unsigned)b, 32 * XI_WARPS, smem, st>>>(xi_grid, d, axis, x, core, sums);
+    const size_t smem = sizeof(float) * 3 * d.nb3;
+    PYL_CHECK_ARG(smem <= 48 * 1024, "grid too large for the shared-memory bins");
+    xi_bin_kernel<<<blocks_of((long long)dims * dims), 256, smem, st>>>(xi_grid, d, axis, sums);
     PYL_LAUNCH_CHECK();
-    xi_row_kernel<<<blocks_of((long long)dims * dims), 256, sizeof(float) * 3 * d.nb3, st>>>(xi_grid, d, axis, core, sums);
+    const long long reps = (long long)sym_groups(dims) * sym_groups(dims);
+    const size_t gsm = 12 * (size_t)d.nb3;
+    const long long b = std::min((reps + 2 * XI_WARPS - 1) / (2 * XI_WARPS), 4LL * num_sms());
+    xi_geometry_kernel<<<(unsigned)b, 32 * XI_WARPS, gsm, st>>>(d, sums);
     PYL_LAUNCH_CHECK();
     return PYL_OK;
 }

@@ -82,3 +82,44 @@ def test_mode_factors_equal_float64(lib, dims, p):
     inner = (kz != 0) & ((kz != dims // 2) | (dims % 2 == 1))      # the other planes keep their Hermitian part
     err = (out.to(torch.complex128) - d)[..., inner].abs()
     assert bool((err <= 2.0 ** -21 * d[..., inner].abs()).all())
+
+
+@pytest.mark.parametrize('dims,axis', [(255, 0), (256, 2), (257, 0), (257, 1), (257, 2), (291, 1), (579, 0)])
+def test_xi_bin_equals_float64_on_larger_sides(lib, dims, axis):
+    test_xi_bin_equals_float64(lib, dims, axis)
+
+
+@pytest.mark.parametrize('dims', [64, 255, 256, 257, 300])
+def test_xi_bin_adds_x_planes_in_float64(lib, dims):
+    """2^24 at (x, y, z) and 1 at (-x, y, z), alone in their bins: the float32 sum of the two
+    loses the 1, the float64 sum of different x planes is exact."""
+    from pylians_gb300._device import ptr, stream_ptr
+    x = torch.zeros((dims,) * 3, device='cuda')
+    bins = []
+    for i in range(4, dims // 2 - 1, 5):
+        x[i, 3, 2] = 2.0 ** 24
+        x[dims - i, 3, 2] = 1.0
+        bins.append(math.isqrt(i * i + 13))
+    assert len(set(bins)) == len(bins)
+    out = torch.empty(lib.load().pyl_xi_sums_len(dims), dtype=torch.float64, device='cuda')
+    lib.call('pyl_xi_bin', ptr(x), dims, 2, ptr(out), stream_ptr())
+    got = out.cpu().numpy()[:3 * (len(out) // 5)].reshape(-1, 3)[bins, 0]
+    assert np.array_equal(got, np.full(len(bins), 2.0 ** 24 + 1.0))
+
+
+@pytest.mark.parametrize('dims', [16, 33, 256, 257])
+def test_xi_bin_lengths_are_float64(lib, dims):
+    """Sums of |r| of the smallest bins: correctly rounded roots (2^-53) and at most one
+    rounding for each of a bin's separations."""
+    from pylians_gb300._device import ptr, stream_ptr
+    x = torch.zeros((dims,) * 3, device='cuda')
+    out = torch.empty(lib.load().pyl_xi_sums_len(dims), dtype=torch.float64, device='cuda')
+    lib.call('pyl_xi_bin', ptr(x), dims, 0, ptr(out), stream_ptr())
+    nb = len(out) // 5
+    R = out.cpu().numpy()[3 * nb:4 * nb]
+    m = range(-4, 5)
+    n2 = [a * a + b * b + c * c for a in m for b in m for c in m]
+    for b in (1, 2, 3):
+        terms = [math.sqrt(v) for v in n2 if b * b <= v < (b + 1) ** 2]
+        ref = math.fsum(terms)
+        assert abs(R[b] - ref) <= (len(terms) + 1) * 2.0 ** -53 * ref
