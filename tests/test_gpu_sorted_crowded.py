@@ -1,0 +1,63 @@
+"""The sorted strategy on particles that leave most of the box empty or crowd a few cells:
+float64 sums of the grids, and times in proportion to those of a uniform box, so that no
+thread is left with work that grows with the empty part or the crowded one.
+
+The bounds on times lie well below what one thread doing such work takes (in brackets)."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+BOX = 1000.0
+
+
+@pytest.fixture(scope='module')
+def MASL():
+    import pylians_gb300.build as b
+    b.build()
+    import pylians_gb300.MAS_library as MASL
+    return MASL
+
+
+def uniform(n, seed=1, part=1.0):
+    g = torch.Generator(device='cuda')
+    g.manual_seed(seed)
+    return torch.rand((n, 3), generator=g, device='cuda') * (BOX * part * (1 - 1e-6))
+
+
+def time_us(MASL, pos, dims, mas, w=None):
+    grid = torch.zeros((dims,) * 3, device='cuda')
+    times = []
+    for _ in range(4):
+        t0, t1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        t0.record()
+        MASL.MA(pos, grid, BOX, mas, w, strategy='sorted')
+        t1.record()
+        torch.cuda.synchronize()
+        times.append(t0.elapsed_time(t1) * 1e3)
+    return min(times[1:])
+
+
+def test_empty_part_of_the_box_costs_nothing(MASL):
+    """512^3, CIC: the particles of an octant (22 times the time of as many all over the
+    box), 1000 in a corner (17 times)."""
+    n = 1 << 22
+    assert time_us(MASL, uniform(n, part=0.5), 512, 'CIC') <= 3.0 * time_us(MASL, uniform(n), 512, 'CIC')
+    assert time_us(MASL, uniform(1000, part=0.01), 512, 'CIC') <= 3.0 * time_us(MASL, uniform(1000), 512, 'CIC')
+
+
+@pytest.mark.parametrize('mas', ['NGP', 'CIC', 'TSC', 'PCS'])
+@pytest.mark.parametrize('dims,lo,hi', [(5, 0.4, 0.6), (8, 0.0, 0.1), (9, 0.9, 0.999), (33, 0.3, 0.4), (64, 0.0, 0.01), (70, 0.99, 0.999)])
+def test_gaps_equal_atomic_sums(MASL, mas, dims, lo, hi):
+    """Columns and segments before, between and after the particles are empty.  Both
+    strategies sum float32 products of the same weights: at most 4000 roundings of 2^-24
+    of a cell's value each."""
+    pos = uniform(4000, seed=dims) * (hi - lo) + lo * BOX
+    w = torch.rand(4000, generator=torch.Generator(device='cuda').manual_seed(7), device='cuda') + 0.5
+    for weights in (None, w):
+        a, b = torch.zeros((dims,) * 3, device='cuda'), torch.zeros((dims,) * 3, device='cuda')
+        MASL.MA(pos, a, BOX, mas, weights, strategy='sorted')
+        MASL.MA(pos, b, BOX, mas, weights, strategy='atomic')
+        x, y = a.cpu().numpy().astype(np.float64), b.cpu().numpy().astype(np.float64)
+        assert np.all(np.abs(x - y) <= 2 * 4000 * 2.0 ** -24 * np.maximum(x, y))
