@@ -93,3 +93,80 @@ def test_ngp_cells_equal_the_serial_sums(MASL, base, counts):
         MASL.MA(torch.from_numpy(pos).cuda(), grid, BOX, 'NGP', None if weights is None else torch.from_numpy(w).cuda(),
                 strategy='sorted')
         assert np.array_equal(grid.cpu().numpy(), ref)
+
+
+def longest_chain(n, s):
+    """Additions that one value passes through at most: 8192 particles of a cell (or their
+    255 companions' share of more) in 32 lanes, the lanes and warps, the particles of s
+    cells that are walked, the s^2 columns, the grid's value."""
+    return 256 + n // 256 + 13 + s * 127 + s * s + 1
+
+
+@pytest.mark.parametrize('mas', ['CIC', 'TSC', 'PCS'])
+@pytest.mark.parametrize('dims,counts', [(1, (300,)), (2, (64, 127, 128, 8192)), (7, (8, 9, 63, 64, 65, 126, 127, 128, 129, 191, 200)),
+                                         (33, (8199, 8200, 8201, 8263, 20000, 1, 500)), (64, tuple(range(60, 140)))])
+def test_crowded_cells_equal_float64(MASL, mas, dims, counts):
+    """Cells of given numbers of particles (around the ends of blocks and the split
+    between a warp and a CTA), the first and the last of the box among them, against
+    float64 sums of the same float32 positions; the same bits on every run."""
+    rng = np.random.default_rng(dims)
+    s = {'CIC': 2, 'TSC': 3, 'PCS': 4}[mas]
+    cells = rng.choice(dims ** 3, min(len(counts), dims ** 3), replace=False)
+    cells[0] = 0
+    cells[-1] = dims ** 3 - 1
+    base = np.concatenate([np.full(k, c) for c, k in zip(cells, counts)])
+    pos = np.stack([base // dims ** 2, base // dims % dims, base % dims], 1) + 0.05 + 0.9 * rng.random((len(base), 3))
+    pos = rng.permutation((pos * (BOX / dims)).astype(np.float32))
+    w = (rng.random(len(pos)) + 0.5).astype(np.float32)
+    for weights in (None, w):
+        grids = []
+        for _ in range(2):
+            a, b = (torch.full((dims,) * 3, 0.5, device='cuda') for _ in range(2))
+            MASL.MA(torch.from_numpy(pos).cuda(), a, BOX, mas, None if weights is None else torch.from_numpy(weights).cuda(),
+                    interlaced=b, strategy='sorted')
+            grids.append((a.cpu().numpy(), b.cpu().numpy()))
+        assert np.array_equal(grids[0], grids[1])
+        for k, shift in ((0, 0.0), (1, 0.5)):
+            x = pos.astype(np.float64) * (dims / BOX) + shift
+            ref = np.full(dims ** 3, 0.5)
+            first, c = [], []
+            for a in range(3):
+                if mas == 'CIC':
+                    f = np.floor(x[:, a])
+                    u = x[:, a] - f
+                    first.append(f), c.append([1 - u, u])
+                elif mas == 'TSC':
+                    f = np.floor(x[:, a] - 0.5)
+                    u = x[:, a] - f - 1
+                    first.append(f), c.append([0.5 * (0.5 - u) ** 2, 0.75 - u * u, 0.5 * (0.5 + u) ** 2])
+                else:
+                    f = np.floor(x[:, a]) - 1
+                    d = [np.abs(x[:, a] - f - j) for j in range(4)]
+                    first.append(f), c.append([np.where(t < 1, (4 - 6 * t * t + 3 * t ** 3) / 6, np.maximum(2 - t, 0) ** 3 / 6) for t in d])
+            for l in range(s):
+                for m in range(s):
+                    for q in range(s):
+                        i = [(first[a] + o).astype(int) % dims for a, o in enumerate((l, m, q))]
+                        v = c[0][l] * c[1][m] * c[2][q]
+                        np.add.at(ref, (i[0] * dims + i[1]) * dims + i[2], v if weights is None else v * weights)
+            # a float32 position is off by 2^-24 of the box, dims * 2^-24 cells, and as much
+            # again in the product and the shift; a weight's slope is at most 1.  The grid's
+            # sum of all particles bounds what that moves in a cell of them.
+            slope = 8.0 * dims * 2.0 ** -24 * 1.5 * s
+            got = grids[0][k].reshape(-1).astype(np.float64)
+            near = np.zeros(dims ** 3)
+            for l in range(s):
+                for m in range(s):
+                    for q in range(s):
+                        i = [(first[a] + o).astype(int) % dims for a, o in enumerate((l, m, q))]
+                        np.add.at(near, (i[0] * dims + i[1]) * dims + i[2], 1.0)
+            tol = (longest_chain(max(counts), s) + 8) * 2.0 ** -24 * ref + slope * near
+            assert np.all(np.abs(got - ref) <= tol)
+
+
+@pytest.mark.parametrize('mas,dims', [('CIC', 128), ('CIC', 256), ('CIC', 512), ('TSC', 256), ('PCS', 256)])
+def test_crowded_cells_cost_little(MASL, mas, dims):
+    """16.8 million particles in a corner of a twentieth of the box's side (walked one by
+    one: 6 to 141 times the time of as many all over the box)."""
+    n = 1 << 24
+    assert time_us(MASL, uniform(n, part=0.05), dims, mas) <= 4.0 * time_us(MASL, uniform(n), dims, mas)
