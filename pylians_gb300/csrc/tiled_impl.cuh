@@ -1228,14 +1228,16 @@ __device__ __forceinline__ void fx_write_out(const unsigned *smw, float *out, co
 }
 
 // Write-out of a bin's part (BinParts): the cells' sums are added to the grid's 64-bit
-// fixed-point words, so the grid does not depend on how the records were divided or in
-// which order the parts end; share_finish_kernel adds the words to the grid.  A part
-// redone in float32 (a cell of 512 or more) goes there in the same units; float sums
-// of weights (any magnitude) and what is not finite go to the grid itself.
+// fixed-point words, so the words do not depend on how the records were divided or in
+// which order the parts end; share_finish_kernel adds them to the grid.  The sums of a part
+// redone in float32 (a cell of 512 or more) go there in the same units, and what is
+// smaller than a unit to the grid itself, so that small cells keep their 24 bits; float
+// sums of weights (any magnitude) and what is not finite go to the grid.
 template <int MAS, bool INTER, bool FLOAT>
 __device__ __forceinline__ void fx_share_out(const unsigned *smw, unsigned long long *share, float *out, const int *o,
                                              int dims, bool interior, float scale, bool weighted)
 {
+    constexpr float UNITS = MAS == PYL_MAS_NGP ? 1.0f : FX_SCALE;   // of 1 (NGP: counts)
     fx_each_cell<MAS, INTER>([&](long long i, int c) {
         const unsigned w = smw[c];
         if (w == 0u) return;
@@ -1243,8 +1245,14 @@ __device__ __forceinline__ void fx_share_out(const unsigned *smw, unsigned long 
             atomicAdd(share + i, (unsigned long long)w);
         } else {
             const float v = __uint_as_float(w);
-            if (!weighted && fabsf(v) < 1e12f) atomicAdd(share + i, (unsigned long long)__float2ll_rn(__fmul_rn(v, FX_SCALE)));
-            else atomicAdd(out + i, __fmul_rn(v, scale));
+            if (!weighted && fabsf(v) < 1e12f) {
+                const long long u = __float2ll_rn(__fmul_rn(v, UNITS));
+                const float rest = __fsub_rn(v, __fmul_rn(__ll2float_rn(u), 1.0f / UNITS));  // exact; 0 from 2 on
+                if (u) atomicAdd(share + i, (unsigned long long)u);
+                if (rest != 0.0f) atomicAdd(out + i, __fmul_rn(rest, scale));
+            } else {
+                atomicAdd(out + i, __fmul_rn(v, scale));
+            }
         }
     }, o, dims, interior);
 }

@@ -85,3 +85,36 @@ def test_batched_parts(mods):
             got = b.grids[s['dims']][s['slot2'] if k else s['slot']].cpu().numpy()
             ref = reference(p, s['dims'], s['MAS'], k) * scale - 1.0
             check(got, ref, scale)
+
+
+@pytest.mark.parametrize('offset', [2.0 ** -5, 2.0 ** -6])
+@pytest.mark.parametrize('mas', ['TSC', 'PCS'])
+def test_small_cells_beside_crowded_ones(mas, offset):
+    """2^18 particles at one point of 64^3 (cells of unit length, so every weight follows
+    from `offset` alone): each part of the bin is redone in float32 for its cells past 512,
+    and the cells of the smallest weights, far below 2^-22, keep float32's relative error,
+    at most one rounding of 2^-24 for each addition and eight for a weight."""
+    import pylians_gb300.build as b
+    b.build()
+    import pylians_gb300.MAS_library as MASL
+    n, dims = 1 << 18, 64
+    o = {'TSC': 0.5, 'PCS': 0.0}[mas] + 1.0 - offset
+    pos = torch.tensor([20.0 + o, 20.0 + o, 20.25], device='cuda').expand(n, 3).contiguous()
+    grid = torch.zeros((dims,) * 3, device='cuda')
+    MASL.MA(pos, grid, float(dims), mas, strategy='tiled')
+    ref = torch.zeros((dims,) * 3, dtype=torch.float64, device='cuda')
+    near = [], [], []
+    for a in range(3):
+        x = float(pos[0, a])
+        for k in range(int(x) - 3, int(x) + 5):
+            s = abs(x - k)
+            if mas == 'TSC':
+                w = 0.75 - s * s if s < 0.5 else 0.5 * max(1.5 - s, 0.0) ** 2
+            else:
+                w = (4 - 6 * s * s + 3 * s ** 3) / 6 if s < 1 else max(2 - s, 0.0) ** 3 / 6
+            near[a].append((k, w))
+    for i, wi in near[0]:
+        for j, wj in near[1]:
+            for k, wk in near[2]:
+                ref[i, j, k] = n * wi * wj * wk
+    assert bool(((grid.double() - ref).abs() <= (n + 24) * 2.0 ** -24 * ref).all())
