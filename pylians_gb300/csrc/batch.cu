@@ -300,11 +300,14 @@ __global__ void __launch_bounds__(256) bt_list_kernel(const pyl_batch_real *__re
     if (per_grid > 1u) {
         if (lane == 0u) shared = atomicAdd(shared_count, grids);
         shared = __shfl_sync(0xffffffffu, shared, 0);
-        if (shared + grids > max_shared) return;            // not reached: see bt_max_shared
     }
+    // no BinShare left (bt_max_shared has one for every bin in parts, unless the items hold more
+    // particles than the caller's total): whole bins, the other parts empty
+    const bool whole = per_grid > 1u && shared + grids > max_shared;
     for (unsigned i = lane; i < n && b + i < max_parts; i += 32) {
         const unsigned first = (i % per_grid) * len, g = i / per_grid;
-        list[b + i] = BtPart{t, (unsigned)real, first, min(len, counts[t] - first), g, per_grid, shared + g, 0u};
+        list[b + i] = whole ? BtPart{t, (unsigned)real, 0u, first ? 0u : counts[t], g, 1u, 0u, 0u}
+                            : BtPart{t, (unsigned)real, first, min(len, counts[t] - first), g, per_grid, shared + g, 0u};
     }
 }
 

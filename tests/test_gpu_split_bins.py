@@ -118,3 +118,28 @@ def test_small_cells_beside_crowded_ones(mas, offset):
             for k, wk in near[2]:
                 ref[i, j, k] = n * wi * wj * wk
     assert bool(((grid.double() - ref).abs() <= (n + 24) * 2.0 ** -24 * ref).all())
+
+
+@pytest.mark.parametrize('interlaced', [False, True])
+def test_batch_of_more_particles_than_the_stated_total(mods, interlaced):
+    """A stated total below the items' particles keeps that many records, in bins whose
+    parts then have no shared words: whole bins.  A particle's weights add up to 1 within
+    27 units of 2^-22."""
+    from pylians_gb300 import _lib
+    from pylians_gb300._device import ptr, stream_ptr
+    _, batch = mods
+    n, total, dims = 400000, 1000, 32
+    g = torch.Generator(device='cuda')
+    g.manual_seed(5)
+    pos = torch.rand((n, 3), generator=g, device='cuda') * (BOX * 0.99)
+    b = batch.RealizationBatch([dict(dims=dims, MAS='TSC', interlaced=interlaced, n=n)], BOX, tune=False, method='tiled')
+    b._tables([pos])
+    b.grids[dims].zero_()
+    nbytes = _lib.load().pyl_ma_batch_tiled_workspace_size(b.total_tiles, total)
+    ws = torch.full((nbytes,), 255, dtype=torch.uint8, device='cuda')
+    _lib.call('pyl_ma_batch_tiled', ptr(b.reals_dev), 1, ptr(b.items_dev), b.n_items, ptr(b.tile_base), b.total_tiles,
+              total, ptr(ws), nbytes, 4, stream_ptr())
+    scale = dims ** 3 / n
+    for k in range(2 if interlaced else 1):
+        got = float(b.grids[dims][b.specs[0]['slot2'] if k else b.specs[0]['slot']].double().sum())
+        assert abs(got - total * scale) <= total * scale * 32 * 2.0 ** -22
