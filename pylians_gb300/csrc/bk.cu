@@ -324,8 +324,8 @@ __global__ void __launch_bounds__(256) shell_sum_kernel(const float2 *__restrict
     }
 }
 
-// The distinct bounds of the shells, ascending; false when they exceed 32 bits (no mode
-// of a grid of at most 4096^3 lies there: 3 * 2048^2 < 2^24).
+// The distinct bounds of the shells, ascending, those past 2^24 as 2^24 (no mode of a
+// grid of at most 4096^3 lies there: 3 * 2048^2 < 2^24).
 void cut_shells(Shells &sh)
 {
     std::vector<int> e;

@@ -1356,6 +1356,7 @@ extern "C" int pyl_pk_bin_batch(const pyl_pk_item *items, int n_items, int dims,
     a.d = d;
     a.rows = nullptr;
     a.items = items;
+    a.low_ctas = 0;
     for (int f = 0; f < MAX_FIELDS; f++) a.mas_p[f] = 0;
     cudaStream_t st = (cudaStream_t)stream;
     const BatchPart bp = batch_part(d, axis, n_items);
