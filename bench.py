@@ -631,7 +631,7 @@ def bench_batch(count, steps=3):
     alg = sum(chain_bytes(s['n'], s['dims'], 2 if s['interlaced'] else 1) for s in specs)
     hbm, src = hbm_peak()
     out = dict(metric='realizations/s', value=count / (ms / 1e3), particles_per_s=npart / (ms / 1e3),
-               ms_per_batch=ms, realizations=count, particles=npart, ctas_per_sm=B.ctas_per_sm,
+               ms_per_batch=ms, realizations=count, particles=npart,
                roofline=dict(alg_bytes=alg, gbs=alg / (ms / 1e3) / 1e9, peak=hbm, peak_source=src,
                              frac=alg / (ms / 1e3) / 1e9 / hbm, unit='GB/s',
                              bytes='sum over realizations of 12 N_p + G (8 N_g + 16 N_h) (chain_bytes)'))

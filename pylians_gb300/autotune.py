@@ -1,6 +1,7 @@
 """Autotuner for the batched deposit: work-item size per realization class and
-CTAs per SM of the persistent launches, for either batch method ('tiled':
-bins + one persistent bin deposit; 'atomic': red.global work queue).
+CTAs per SM of the persistent launch of the 'atomic' method (red.global work
+queue); the launches of the 'tiled' one (bins + one persistent bin deposit) have
+fixed grids.
 
 Classes are (grid side, particle-count bucket (power of 2), MAS, interlaced).
 For a class the tuner deposits one synthetic realization of that class through
@@ -126,6 +127,8 @@ def item_size(dims, n, MAS, interlaced, tune=True, method='atomic'):
 
 
 def ctas_per_sm(tune=True, method='atomic'):
+    if method == 'tiled':                   # no launch of pyl_ma_batch_tiled depends on it
+        return DEFAULT_CTAS
     key = '%s/%s/ctas_per_sm' % (_device_key(), method)
     with _lock:
         c = _load()
@@ -133,8 +136,7 @@ def ctas_per_sm(tune=True, method='atomic'):
             return int(c[key])
         if not tune:
             return DEFAULT_CTAS
-        cands = CTA_CANDIDATES if method == 'atomic' else (1, 2)     # tiled kernels run 1024 threads per CTA
-        best = min(cands, key=lambda k: _time_deposit(128, 1 << 22, 'CIC', True, DEFAULT_ITEM, k, method=method))
+        best = min(CTA_CANDIDATES, key=lambda k: _time_deposit(128, 1 << 22, 'CIC', True, DEFAULT_ITEM, k, method=method))
         c[key] = int(best)
         _save()
         return int(best)

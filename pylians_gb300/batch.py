@@ -33,7 +33,8 @@ PK_ITEM_DT = np.dtype([('dk', '<u8'), ('dk2', '<u8'), ('sums', '<u8'), ('mas_p',
 
 
 class RealizationBatch(object):
-    """specs: list of dicts with keys dims, MAS, interlaced, n (particle count)."""
+    """specs: list of dicts with keys dims, MAS, interlaced, n (particle count).
+    ctas_per_sm (1..8; None: tuned) is the atomic method's; the tiled one ignores it."""
 
     def __init__(self, specs, BoxSize, axis=0, device=None, tune=True, ctas_per_sm=None, order='size',
                  method='auto'):

@@ -62,3 +62,10 @@ def test_unreadable_cache_starts_empty(tuner):
     path.write_text('{not json')
     assert at_.item_size(64, 5000, 'PCS', False, tune=False) == at_.DEFAULT_ITEM
     assert at_._cache == {}
+
+
+def test_tiled_launches_are_not_timed_for_ctas(tuner):
+    """pyl_ma_batch_tiled's grids are fixed: there is no choice to time or to keep."""
+    at_, path, timed = tuner
+    assert at_.ctas_per_sm(method='tiled') == at_.DEFAULT_CTAS
+    assert not timed and not path.exists()
