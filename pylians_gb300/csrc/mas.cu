@@ -152,15 +152,19 @@ int launch_atomic(const float *pos, const float *w, long long n, float *grid, fl
 
 // ------------------------------------------------------------------ NGP counts
 // Unweighted NGP on grids that stay in L2: whole-number counts by red.global, a run of
-// lanes in one cell as one addition, then one pass adds them to the grids: the bits of the
-// tiled deposit, which rounds a cell's total once too.  Bound by the additions in L2; with
+// lanes in one cell as one addition, then one pass adds them to the grids, rounding a
+// cell's total once: on grids of whole numbers the bits of the tiled deposit (which adds a
+// bin's edge cells of the shifted grid in two parts).  Bound by the additions in L2; with
 // one addition a particle the tiled deposit's passes (count, placement, deposit) cost more.
 // Particles in no order, counts and tiled (us):
 //   256^3 particles: 64^3 122 and 855, 128^3 126 and 337, 256^3 184 and 318; interlaced
 //   200^3 234 and 474;  400^3 on 128^3 373 and 1121;  2^20 on 256^3 83 and 84.
 // Past NGP_COUNT_BYTES the counts leave L2 (256^3 interlaced, 128 MB: 587 us without their
 // passes, 466 tiled), and past NGP_COUNT_PER_CELL the additions to one cell queue (400^3 on 16^3:
-// 1470 and 1353).
+// 1470 and 1353).  Lanes of one cell that do not follow each other are added together where
+// a lane's cell is also that of one 9 or 16 lanes away, the sign of few cells in no order:
+// 256^3 particles at 4 points of 128^3 3825 -> 674 us (1923 tiled), 16 points 1239 -> 695
+// (1074); a match in every warp would take 200 us for the 126 of uniform particles.
 template <bool INTERLACED>
 __global__ void __launch_bounds__(256) ngp_count_kernel(const float *__restrict__ pos, long long n, int dims, float inv,
                                                         float halfcell, unsigned *__restrict__ cnt,
@@ -185,7 +189,15 @@ __global__ void __launch_bounds__(256) ngp_count_kernel(const float *__restrict_
         const unsigned prev = __shfl_up_sync(0xffffffffu, cell, 1);
         const bool head = lane == 0 || cell != prev;
         const unsigned heads = __ballot_sync(0xffffffffu, head), after = heads & ~((2u << lane) - 1u);
-        if (head && valid) atomicAdd((g == 0 ? cnt : cnt2) + cell, (unsigned)((after ? __ffs(after) - 1 : 32) - lane));
+        unsigned adds = (unsigned)((after ? __ffs(after) - 1 : 32) - lane);
+        bool first = head;
+        const unsigned far16 = __shfl_xor_sync(0xffffffffu, cell, 16), far9 = __shfl_xor_sync(0xffffffffu, cell, 9);
+        if (__any_sync(0xffffffffu, cell == far16 || cell == far9) && __popc(heads) > 4) {
+            const unsigned peers = __match_any_sync(0xffffffffu, cell);
+            first = lane == __ffs(peers) - 1;
+            adds = (unsigned)__popc(peers);
+        }
+        if (first && valid) atomicAdd((g == 0 ? cnt : cnt2) + cell, adds);
     }
 }
 
