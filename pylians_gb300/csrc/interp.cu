@@ -57,15 +57,27 @@ __device__ __forceinline__ float cic_at(const float *__restrict__ g, int dims, f
     return cic_value(g, dims, inv, [&](int a) { return __ldg(q + a); });
 }
 
-// A particle a thread and no resident grid with a stride: CTAs that start in order keep
-// ordered particles together in L2 (256^3 in lattice order on 512^3: 341 -> 240 us).
+// Four particles a thread, a grid's width apart: CTAs that start in order keep ordered
+// particles together in L2, where a resident grid of threads drifts apart, and a CTA for
+// every 256 particles costs more than they do (256^3 particles, resident / 4 / 1 each, us:
+// lattice, x slowest, on 256^3 115, 113, 130, on 320^3 120, 117, 135, on 512^3 145, 141, 151;
+// z slowest on 400^3 545, 455, 450, on 512^3 1382, 1286, 1219; no order on 512^3 1230, 1221, 1208).
+constexpr int IP_PER_THREAD = 4;
+
+__device__ __forceinline__ void interp_direct(const float *__restrict__ g, int dims, float inv,
+                                              const float *__restrict__ pos, long long n, float *__restrict__ den,
+                                              unsigned ctas)
+{
+    const long long stride = (long long)ctas * blockDim.x;
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride)
+        den[i] = cic_at(g, dims, inv, pos + 3 * i);
+}
+
 __global__ void __launch_bounds__(256) cic_interp_kernel(const float *__restrict__ g, int dims, float inv,
                                                          const float *__restrict__ pos, long long n,
                                                          float *__restrict__ den)
 {
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride)
-        den[i] = cic_at(g, dims, inv, pos + 3 * i);
+    interp_direct(g, dims, inv, pos, n, den, gridDim.x);
 }
 
 // ---- interpolation by slabs ----------------------------------------------------------
@@ -217,12 +229,11 @@ __global__ void __launch_bounds__(IT_THREADS, 3) interp_split_kernel(const float
 // (a resident grid with a stride drifts apart over the slabs: 590 us for 310).
 __global__ void __launch_bounds__(256) interp_slab_kernel(const float *__restrict__ g, int dims, float inv,
                                                           const float *__restrict__ pos, long long n, Slabs sl, int tiles,
-                                                          int width, InterpWs ws, float *__restrict__ den)
+                                                          int width, unsigned direct_ctas, InterpWs ws, float *__restrict__ den)
 {
     const long long first = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (!*ws.scattered) {
-        for (long long i = first; i < n; i += (long long)gridDim.x * blockDim.x)
-            den[i] = cic_at(g, dims, inv, pos + 3 * i);
+        if (blockIdx.x < direct_ctas) interp_direct(g, dims, inv, pos, n, den, direct_ctas);
         return;
     }
     const long long job = first / width;
@@ -268,21 +279,21 @@ inline unsigned blocks_of(long long n)
     return (unsigned)(b < 1 ? 1 : (b > cap ? cap : b));
 }
 
+// CTAs of interp_direct: IP_PER_THREAD particles a thread, fewer where that leaves SMs idle.
+inline unsigned direct_blocks(long long n)
+{
+    const long long per_cta = 256 * IP_PER_THREAD;
+    return std::max(blocks_of(n), (unsigned)std::min((n + per_cta - 1) / per_cta, 1ll << 30));
+}
+
 }  // namespace
 }  // namespace pyl
 
 using namespace pyl;
 
-// Measured with 256^3 particles, in no order / on a lattice, z slowest / x slowest (us):
-//   up to INTERP_CACHED bytes of grid a resident grid of threads (cic_interp_kernel) beats
-//   one thread per particle for ordered particles: 128^3 113 and 127, 256^3 134 and 140;
-//   past it the latter does: 512^3 285 and 246, 1024^3 1100 and 607;
-//   slabs, thread per particle: 320^3 449, 588 / 447, 298 / 181, 177; 400^3 447, 965 / 404, 410 /
-//   208, 212; 512^3 449, 1221 / 416, 697 / 240, 246; 1024^3 778, 1540 / 781, 1387 / 621, 607.
-// The lattice with x slowest pays the sample and two empty kernels, 10 us: from INTERP_MIN_N
-// particles on little beside the rest (4,000,000 on 512^3: 122 and 107 us, 8,000,000: 156 and
-// 145, both below a resident grid's 117 and 162).
-constexpr long long INTERP_CACHED = 96ll << 20;
+// Slabs and direct, 256^3 particles in no order / sorted by z (us): 320^3 449, 578 / -, 450; 400^3
+// 442, 960 / 484, 573; 512^3 446, 1221 / 589, 1163; 640^3 478, 1429 / 602, 1440.  Ordered particles pay
+// the sample and two empty kernels, 9 to 13 us of 137 (256^3, lattice on 400^3) or of 87 (204^3).
 constexpr long long INTERP_MIN_BYTES = 240ll << 20;
 constexpr long long INTERP_MIN_N = 1ll << 23;
 
@@ -318,8 +329,9 @@ extern "C" int pyl_cic_interp_slabs(const float *grid, int dims, float box_size,
                                                                                              tiles, sl, ws);
         PYL_LAUNCH_CHECK();
         const long long threads = (long long)sl.count * tiles * width;
-        interp_slab_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(grid, dims, inv, pos + 3 * done, len, sl, tiles,
-                                                                              width, ws, out + done);
+        const unsigned direct = direct_blocks(len);
+        interp_slab_kernel<<<std::max((unsigned)((threads + 255) / 256), direct), 256, 0, st>>>(
+            grid, dims, inv, pos + 3 * done, len, sl, tiles, width, direct, ws, out + done);
         PYL_LAUNCH_CHECK();
         interp_place_kernel<<<std::min(tiles, 4 * num_sms()), IT_THREADS, 0, st>>>(ws, sl.count, tiles, out + done);
         PYL_LAUNCH_CHECK();
@@ -336,9 +348,7 @@ extern "C" int pyl_cic_interp(const float *grid, int dims, float box_size, const
     PYL_CHECK_ARG(box_size > 0.0f && isfinite(box_size), "BoxSize must be positive and finite");
     if (n == 0) return PYL_OK;
     const float inv = (float)dims / box_size;             // MAS_library.pyx:575
-    const bool cached = 4ll * dims * dims * dims <= INTERP_CACHED;
-    const unsigned blocks = cached ? blocks_of(n) : (unsigned)std::min<long long>((n + 255) / 256, 1ll << 30);
-    cic_interp_kernel<<<blocks, 256, 0, (cudaStream_t)stream>>>(grid, dims, inv, pos, n, out);
+    cic_interp_kernel<<<direct_blocks(n), 256, 0, (cudaStream_t)stream>>>(grid, dims, inv, pos, n, out);
     PYL_LAUNCH_CHECK();
     return PYL_OK;
 }
