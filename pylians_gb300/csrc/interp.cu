@@ -87,9 +87,9 @@ __global__ void __launch_bounds__(256) cic_interp_kernel(const float *__restrict
 //      each) and writes them with their places;
 //   2. interp_slab_kernel takes slab after slab, the particles of all tiles, from L2;
 //   3. interp_place_kernel puts each tile's values back into the particles' order.
-// Whether the particles are in no order is read off a sample (interp_scattered); else the
-// second kernel interpolates them as cic_interp_kernel does and the others have nothing to
-// do.  The same bits either way: every value comes from cic_value.
+// Whether the particles are in no order, over more of the grid than stays in L2, is read off
+// a sample (interp_scattered); else the second kernel interpolates them as
+// cic_interp_kernel does and the others have nothing to do.  The same bits either way: every value comes from cic_value.
 // 256^3 particles in no order on 512^3: 1250 -> 449 us (split 102, slabs 311, places 27).  The
 // slabs' kernel is bound by the random loads in L1 and L2 (87 and 78 % of their throughput;
 // 8 loads of 12 wavefronts, 94 million sectors); a grid that fits L2 takes as long (322 at
@@ -135,27 +135,52 @@ inline InterpWs interp_layout(void *base, long long n, int dims)
 constexpr size_t INTERP_SMEM = (size_t)IT * 14 + sizeof(unsigned) * IS_MAX;
 
 // True where IT consecutive particles lie, as a rule, in more than half of the slabs that
-// as many particles in no order would: 64 of each of 16 tiles, one tile a warp, at hashed
-// places (a lattice's rows have a period).  Every CTA comes to the same answer.
+// as many particles in no order would, and all of them in a part of the grid of more than
+// INTERP_PART bytes: 64 of each of 16 tiles, one tile a warp, at hashed places (a lattice's
+// rows have a period); the part is the share of 8^3 cells of the box that hold particles,
+// by how many of them hold one of 512.  (256^3 particles in one octant, direct
+// and by slabs: 400^3 302 and 442 us, 450^3 308 and 441, 512^3 609 and 439.)  Every CTA comes
+// to the same answer.
+constexpr float INTERP_PART = 56.0f * (1 << 20);
+
 __device__ bool interp_scattered(const float *__restrict__ pos, long long n, int dims, float inv, Slabs sl)
 {
-    __shared__ unsigned seen[IT_THREADS / 32][IS_MAX / 32];
+    __shared__ unsigned seen[IT_THREADS / 32][IS_MAX / 32], boxes[16];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const long long span = min((long long)IT, n), base = (n - span) / (IT_THREADS / 32) * warp;
-    float x[2];
-#pragma unroll
-    for (int j = 0; j < 2; j++) x[j] = __ldg(pos + 3 * (base + ((threadIdx.x * 2 + j) * 2654435769u >> 20) % span));
-    if (lane < IS_MAX / 32) seen[warp][lane] = 0;
-    __syncwarp();
+    const unsigned span = (unsigned)min((long long)IT, n);
+    const float *tile = pos + 3 * ((n - span) / (IT_THREADS / 32) * warp);
+    unsigned at[2];
 #pragma unroll
     for (int j = 0; j < 2; j++) {
-        const unsigned b = (unsigned)wrap_index(__float2int_rz(truncf(__fmul_rn(x[j], inv))), dims) / (unsigned)sl.planes;
+        at[j] = (threadIdx.x * 2 + j) * 2654435769u >> 20;                      // below IT
+        if (span < IT) at[j] %= span;
+    }
+    const float x[2] = {__ldg(tile + 3 * at[0]), __ldg(tile + 3 * at[1])};
+    const float y = __ldg(tile + 3 * at[0] + 1), z = __ldg(tile + 3 * at[0] + 2);
+    if (lane < IS_MAX / 32) seen[warp][lane] = 0;
+    if (threadIdx.x < 16) boxes[threadIdx.x] = 0;
+    __syncthreads();
+    auto cell = [&](float p) { return (unsigned)wrap_index(__float2int_rz(truncf(__fmul_rn(p, inv))), dims); };
+    auto eighth = [&](unsigned k) { return min(7u, (unsigned)(k * (8.0f / dims))); };
+    const unsigned k[2] = {cell(x[0]), cell(x[1])};
+#pragma unroll
+    for (int j = 0; j < 2; j++) {
+        const unsigned b = k[j] / (unsigned)sl.planes;
         atomicOr(&seen[warp][b / 32], 1u << (b % 32));
     }
+    const unsigned box = (8 * eighth(k[0]) + eighth(cell(y))) * 8 + eighth(cell(z));
+    atomicOr(&boxes[box / 32], 1u << (box % 32));
     __syncwarp();
     const int used = __reduce_add_sync(~0u, lane < IS_MAX / 32 ? __popc(seen[warp][lane]) : 0);
     const float fresh = sl.count * (1.0f - __expf(-64.0f / sl.count));
-    return __syncthreads_count(2 * used > fresh) > IT_THREADS / 2;
+    const bool mixed = __syncthreads_count(2 * used > fresh) > IT_THREADS / 2;
+    int held = 0;
+#pragma unroll
+    for (int i = 0; i < 16; i++) held += __popc(boxes[i]);
+    float boxed = (float)held;                               // of them, m (1 - exp(-512 / m)) hold one
+#pragma unroll
+    for (int i = 0; i < 3; i++) boxed = held / (1.0f - __expf(-512.0f / boxed));
+    return mixed && boxed * (4.0f / 512.0f) * dims * dims * dims > INTERP_PART;
 }
 
 __global__ void __launch_bounds__(IT_THREADS, 3) interp_split_kernel(const float *__restrict__ pos, long long n,
