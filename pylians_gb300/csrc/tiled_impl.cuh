@@ -1568,7 +1568,8 @@ int launch_deposit_fx(const TiledWs &ws, TileGeom g, float inv, float halfcell, 
             const size_t bytes = bin_share_bytes(ws.n, MAS, g.dims, I);
             if (bytes) {
                 share = (unsigned long long *)ws.halo;
-                kern = bin_deposit_fx_tma_kernel<MAS, I, RR, false, false, false, true>;
+                kern = tot ? bin_deposit_fx_tma_kernel<MAS, I, RR, false, true, false, true>
+                           : bin_deposit_fx_tma_kernel<MAS, I, RR, false, false, false, true>;
                 PYL_CUDA(cudaMemsetAsync(share, 0, bytes, st));
             }
         }
