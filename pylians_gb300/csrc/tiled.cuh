@@ -178,7 +178,11 @@ inline size_t owned_halo_floats(int mas, int dims, bool inter)
 // idle when a CTA takes a whole bin: its records then go to several CTAs, which add
 // their cells to 64-bit fixed-point words of the grid.  A part is an eighth of an SM's
 // share of all records, and at least PART_ADDS corner additions, with four times the
-// parts of an average bin for the heavier ones (the last part takes what is left).
+// parts of an average bin for the heavier ones (the last part takes what is left).  An
+// average bin of less than two parts stays whole: its longest part takes as long, and the
+// words are zeroed and added besides (2^22 particles on 128^3, CIC interlaced, one part a
+// bin: whole 197 us, parts 235; 2^20 on 64^3, CIC: 144 and 156; interlaced, two parts a bin: 254
+// and 184).
 // Whole bins and parts measured: 512^3 particles on 64^3, PCS interlaced (8 bins, cells
 // past 512 that send whole bins to float32 sums): 1236 and 11.8 ms; 400^3 with masses on
 // 100^3, CIC (64 bins): 4.49 and 1.89; 256^3 on 128^3, CIC interlaced (64 bins): 0.58 and
@@ -194,7 +198,7 @@ inline BinParts bin_parts(long long n, int mas, int dims, bool inter)
     const int S = mas == PYL_MAS_NGP ? 1 : mas;
     const long long adds = (long long)S * S * S * (inter ? 2 : 1);
     const long long len = std::max((n + share - 1) / share, PART_ADDS / adds);
-    if (2 * bins > num_sms() || n / bins < len) return BinParts{0u, 1u};
+    if (2 * bins > num_sms() || n / bins < 2 * len) return BinParts{0u, 1u};
     return BinParts{(unsigned)len, (unsigned)std::min(4 * (n / bins / len + 1), 65535LL)};
 }
 

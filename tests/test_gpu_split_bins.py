@@ -170,3 +170,15 @@ def test_crowded_cells_of_parts_cost_little(mods):
             times.append(t0.elapsed_time(t1))
         best.append(min(times[1:]))
     assert best[1] <= 1.6 * best[0]
+
+
+@pytest.mark.parametrize('dims,mas,inter,parts', [(128, 2, 1, 16), (64, 2, 0, 8), (64, 4, 1, 128)])
+def test_average_bins_of_less_than_two_parts_stay_whole(mods, dims, mas, inter, parts):
+    """The workspace has room for the grids' words only from two parts (of 2^20 additions,
+    `parts` a particle) an average bin on."""
+    from pylians_gb300 import _lib
+    size = _lib.load().pyl_ma_workspace_size
+    bins, n = (dims // 32) ** 3, 2 * (dims // 32) ** 3 * (1 << 20) // parts
+    words = 8 * dims ** 3 * (2 if inter else 1)
+    assert size(n, 3, dims, mas, 2, inter) - size(n - bins, 3, dims, mas, 2, inter) >= words
+    assert size(n - bins, 3, dims, mas, 2, inter) - size(n - 2 * bins, 3, dims, mas, 2, inter) < words // 4
