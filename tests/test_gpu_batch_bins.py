@@ -25,3 +25,33 @@ def test_ngp_counts(dims):
         got = (B.grids[dims][i].cpu().numpy().astype(np.float64).ravel() + 1.0) * s['n'] / dims ** 3
         # overdensity = count * dims^3 / n - 1 in float32: one rounding of the product, one of the sum
         assert np.abs(got - ref).max() <= 2.0 ** -23 * max(1.0, ref.max())
+
+
+def test_few_large_items_are_divided():
+    """Two realizations of 3 million particles in items of 65536 (92 of them) take little
+    more than in items of 4096 (1.6 times with an item to a CTA), and give the same counts."""
+    import pylians_gb300.build as b
+    b.build()
+    from pylians_gb300 import batch
+    dims, n = 128, 3000000
+    g = torch.Generator(device='cuda')
+    g.manual_seed(1)
+    pos = [torch.rand((n, 3), generator=g, device='cuda') * (dims - 0.01) for _ in range(2)]
+    times, grids = [], []
+    for item in (4096, 65536):
+        B = batch.RealizationBatch([dict(dims=dims, MAS='NGP', interlaced=False, n=n)] * 2, float(dims), method='tiled',
+                                   tune=False)
+        B.item_sizes = [item] * 2
+        t = []
+        for _ in range(5):
+            t0, t1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            t0.record()
+            for _ in range(4):
+                B.step(pos)
+            t1.record()
+            torch.cuda.synchronize()
+            t.append(t0.elapsed_time(t1))
+        times.append(min(t))
+        grids.append(B.grids[dims].clone())
+    assert torch.equal(*grids)
+    assert times[1] <= 1.25 * times[0]
