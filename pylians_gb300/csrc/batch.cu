@@ -97,7 +97,7 @@ __global__ void __launch_bounds__(256) scale_value_kernel(float *g, long long n,
 //   bt_place:   persistent over the items: per 4096-particle batch, shared-memory
 //               ranks per bin, one global atomic per bin to reserve a range,
 //               records (x, y, z, 1) written into their bins' ranges;
-//   bt_adds, bt_parts, bt_list: the deposit's work list: every bin of every grid (the
+//   bt_list:    the deposit's work list: every bin of every grid (the
 //               interlaced one apart), those of more than a quarter of an SM's share
 //               of all corner additions in parts of that size (BinShare), so that
 //               the crowded bins of a small grid (7.9 million particles in the 8 bins
@@ -185,10 +185,17 @@ __device__ __forceinline__ void load_quad(const float *pos, long long q, long lo
     }
 }
 
+__host__ __device__ inline unsigned bt_corners(int mas)
+{
+    const unsigned s = mas == PYL_MAS_NGP ? 1u : (unsigned)mas;
+    return s * s * s;
+}
+
 __global__ void __launch_bounds__(BT_THREADS, BT_CTAS) bt_count_kernel(const pyl_batch_real *__restrict__ reals,
                                                         const pyl_batch_item *__restrict__ items, int n_items, int split,
                                                         const unsigned *__restrict__ tile_base,
-                                                        unsigned *__restrict__ counts, unsigned *counter)
+                                                        unsigned *__restrict__ counts, unsigned long long *adds,
+                                                        unsigned *counter)
 {
     __shared__ unsigned h[BT_MAX_TILES];
     __shared__ int cur;
@@ -216,17 +223,13 @@ __global__ void __launch_bounds__(BT_THREADS, BT_CTAS) bt_count_kernel(const pyl
                 if (q + u < end) atomicAdd(h + bt_key_rt(r.mas, p[u], r.inv, r.dims, nt), 1u);
         }
         __syncthreads();
+        if (threadIdx.x == 0 && item.count)
+            atomicAdd(adds, (unsigned long long)item.count * bt_corners(r.mas) * (r.grid_interlaced ? 2u : 1u));
         const unsigned base = tile_base[item.real];
         for (int t = threadIdx.x; t < ntiles; t += blockDim.x)
             if (h[t]) atomicAdd(counts + base + t, h[t]);
         __syncthreads();
     }
-}
-
-__host__ __device__ inline unsigned bt_corners(int mas)
-{
-    const unsigned s = mas == PYL_MAS_NGP ? 1u : (unsigned)mas;
-    return s * s * s;
 }
 
 // Parts of a batch of `adds` corner additions: at most BT_PARTS_PER_SM an SM, none below
@@ -274,65 +277,55 @@ __device__ __forceinline__ int bt_real_of(const unsigned *__restrict__ tile_base
     return lo;
 }
 
-// Corner additions of the whole batch.
-__global__ void __launch_bounds__(256) bt_adds_kernel(const pyl_batch_real *__restrict__ reals, int n_reals,
-                                                      const unsigned *__restrict__ tile_base, unsigned total_tiles,
-                                                      const unsigned *__restrict__ counts, unsigned long long *adds)
-{
-    const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
-    unsigned long long a = 0;
-    if (t < total_tiles) {
-        const pyl_batch_real &r = reals[bt_real_of(tile_base, n_reals, t)];
-        a = (unsigned long long)counts[t] * bt_corners(r.mas) * (r.grid_interlaced ? 2u : 1u);
-    }
-    for (int o = 16; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
-    if ((threadIdx.x & 31) == 0 && a) atomicAdd(adds, a);
-}
-
-// Parts of each bin.
-__global__ void __launch_bounds__(256) bt_parts_kernel(const pyl_batch_real *__restrict__ reals, int n_reals,
-                                                       const unsigned *__restrict__ tile_base, unsigned total_tiles,
-                                                       const unsigned *__restrict__ counts,
-                                                       const unsigned long long *__restrict__ adds, unsigned sms,
-                                                       unsigned *__restrict__ parts)
-{
-    const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= total_tiles) return;
-    const pyl_batch_real &r = reals[bt_real_of(tile_base, n_reals, t)];
-    const unsigned len = bt_part_len(*adds, sms, r.mas);
-    parts[t] = (counts[t] / len + (counts[t] % len != 0u)) * (r.grid_interlaced ? 2u : 1u);
-}
-
-// The work list, in bin order: a bin's parts of the plain grid, then of the interlaced
-// one.  Each grid's bin in parts takes a BinShare.
+// The work list: a bin's parts of the plain grid, then of the interlaced one, bins in any
+// order (a warp reserves the places of its 32 bins).  Each grid's bin in parts takes a
+// BinShare.  With kernels of their own for the sum of additions, the parts of each bin and
+// their scan, four realizations of 512^3 took 27 us longer, one of 64^3 8.
 __global__ void __launch_bounds__(256) bt_list_kernel(const pyl_batch_real *__restrict__ reals, int n_reals,
                                                       const unsigned *__restrict__ tile_base, unsigned total_tiles,
                                                       const unsigned *__restrict__ counts,
                                                       const unsigned long long *__restrict__ adds, unsigned sms,
-                                                      const unsigned *__restrict__ first_part, unsigned max_parts,
-                                                      unsigned max_shared, unsigned *shared_count,
-                                                      BtPart *__restrict__ list)
+                                                      unsigned max_parts, unsigned max_shared, unsigned *n_parts,
+                                                      unsigned *shared_count, BtPart *__restrict__ list)
 {
-    const unsigned t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);      // a warp per bin
-    const unsigned lane = threadIdx.x & 31u;
-    if (t >= total_tiles) return;
-    const unsigned b = first_part[t], n = first_part[t + 1] - b;
-    if (n == 0u) return;
-    const int real = bt_real_of(tile_base, n_reals, t);
-    const unsigned len = bt_part_len(*adds, sms, reals[real].mas), grids = reals[real].grid_interlaced ? 2u : 1u;
-    const unsigned per_grid = n / grids;
-    unsigned shared = 0u;
-    if (per_grid > 1u) {
-        if (lane == 0u) shared = atomicAdd(shared_count, grids);
-        shared = __shfl_sync(0xffffffffu, shared, 0);
+    const unsigned t = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31u;
+    unsigned count = 0u, real = 0u, len = 1u, grids = 1u, parts = 0u, shared = 0u;
+    if (t < total_tiles) {
+        count = counts[t];
+        real = (unsigned)bt_real_of(tile_base, n_reals, t);
+        len = bt_part_len(*adds, sms, reals[real].mas);
+        grids = reals[real].grid_interlaced ? 2u : 1u;
+        parts = count / len + (count % len != 0u);          // of each grid
     }
+    unsigned end = parts * grids;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned v = __shfl_up_sync(0xffffffffu, end, o);
+        if (lane >= (unsigned)o) end += v;
+    }
+    const unsigned total = __shfl_sync(0xffffffffu, end, 31);
+    if (total == 0u) return;
+    unsigned first = 0u;
+    if (lane == 0u) first = atomicAdd(n_parts, total);
+    first = __shfl_sync(0xffffffffu, first, 0) + end - parts * grids;
+    if (parts > 1u) shared = atomicAdd(shared_count, grids);
     // no BinShare left (bt_max_shared has one for every bin in parts, unless the items hold more
     // particles than the caller's total): whole bins, the other parts empty
-    const bool whole = per_grid > 1u && shared + grids > max_shared;
-    for (unsigned i = lane; i < n && b + i < max_parts; i += 32) {
-        const unsigned first = (i % per_grid) * len, g = i / per_grid;
-        list[b + i] = whole ? BtPart{t, (unsigned)real, 0u, first ? 0u : counts[t], g, 1u, 0u, 0u}
-                            : BtPart{t, (unsigned)real, first, min(len, counts[t] - first), g, per_grid, shared + g, 0u};
+    const bool whole = parts > 1u && shared + grids > max_shared;
+    auto entry = [&](unsigned i, unsigned tile, unsigned r, unsigned n, unsigned l, unsigned per_grid, unsigned sh, bool w) {
+        const unsigned from = (i % per_grid) * l, g = i / per_grid;
+        return w ? BtPart{tile, r, 0u, from ? 0u : n, g, 1u, 0u, 0u} : BtPart{tile, r, from, min(l, n - from), g, per_grid, sh + g, 0u};
+    };
+    if (parts == 1u)
+        for (unsigned i = 0; i < grids && first + i < max_parts; i++) list[first + i] = entry(i, t, real, count, len, 1u, 0u, false);
+    for (unsigned many = __ballot_sync(0xffffffffu, parts > 1u); many; many &= many - 1u) {
+        const int s = __ffs(many) - 1;                       // bins in parts: a warp for each
+        const unsigned b = __shfl_sync(0xffffffffu, first, s), p = __shfl_sync(0xffffffffu, parts, s);
+        const unsigned n = __shfl_sync(0xffffffffu, p * grids, s), r = __shfl_sync(0xffffffffu, real, s);
+        const unsigned c = __shfl_sync(0xffffffffu, count, s), l = __shfl_sync(0xffffffffu, len, s);
+        const unsigned sh = __shfl_sync(0xffffffffu, shared, s), tile = __shfl_sync(0xffffffffu, t, s);
+        const bool w = __shfl_sync(0xffffffffu, (int)whole, s) != 0;
+        for (unsigned i = lane; i < n && b + i < max_parts; i += 32) list[b + i] = entry(i, tile, r, c, l, p, sh, w);
     }
 }
 
@@ -345,7 +338,7 @@ __global__ void __launch_bounds__(256) bt_share_zero_kernel(const unsigned *__re
     for (size_t i = blockIdx.x * blockDim.x + threadIdx.x; i < BT_SHARE_CELLS; i += gridDim.x * blockDim.x) z[i] = 0ull;
 }
 
-// Exclusive scan of n counts into offsets[0..n] and (where given) cursor[0..n), one CTA.
+// Exclusive scan of n counts into offsets[0..n] and cursor[0..n), one CTA.
 __global__ void __launch_bounds__(1024) bt_scan_kernel(const unsigned *__restrict__ counts, unsigned n,
                                                        unsigned *__restrict__ offsets, unsigned *__restrict__ cursor)
 {
@@ -365,7 +358,7 @@ __global__ void __launch_bounds__(1024) bt_scan_kernel(const unsigned *__restric
     unsigned long long run = part[threadIdx.x] - sum;
     for (unsigned i = b; i < e; i++) {
         offsets[i] = (unsigned)run;
-        if (cursor) cursor[i] = (unsigned)run;
+        cursor[i] = (unsigned)run;
         run += counts[i];
     }
     if (threadIdx.x == blockDim.x - 1) offsets[n] = (unsigned)part[threadIdx.x];
@@ -631,7 +624,7 @@ __global__ void __launch_bounds__(1024) bt_deposit_kernel(const pyl_batch_real *
 }
 
 struct BtWs {
-    unsigned *counts, *offsets, *cursor, *counters, *parts, *first_part, *done;
+    unsigned *counts, *offsets, *cursor, *counters, *done;
     unsigned long long *adds, *share;
     BtPart *list;
     float4 *rec;
@@ -648,16 +641,15 @@ BtWs bt_layout(void *base, unsigned total_tiles, long long total_particles)
     w.counts = (unsigned *)(b + o); o = bt_align(o + 4 * ((size_t)total_tiles + 1));
     w.offsets = (unsigned *)(b + o); o = bt_align(o + 4 * ((size_t)total_tiles + 1));
     w.cursor = (unsigned *)(b + o); o = bt_align(o + 4 * ((size_t)total_tiles + 1));
-    // counters, the count of additions and the parts' arrivals: zeroed together
+    // counters (of items, parts and BinShares), the count of additions and the parts'
+    // arrivals: zeroed together
     const size_t shared = bt_max_shared(total_tiles, total_particles);
     w.counters = (unsigned *)(b + o);
-    w.adds = (unsigned long long *)(b + o + 16);
+    w.adds = (unsigned long long *)(b + o + 24);
     w.done = (unsigned *)(b + o + 32);
     w.zero_bytes = 32 + 4 * shared;
     o = bt_align(o + w.zero_bytes);
     w.share = (unsigned long long *)(b + o); o = bt_align(o + 8 * BT_SHARE_CELLS * shared);
-    w.parts = (unsigned *)(b + o); o = bt_align(o + 4 * ((size_t)total_tiles + 1));
-    w.first_part = (unsigned *)(b + o); o = bt_align(o + 4 * ((size_t)total_tiles + 1));
     w.list = (BtPart *)(b + o); o = bt_align(o + sizeof(BtPart) * bt_max_parts(total_tiles));
     w.rec = (float4 *)(b + o); o = bt_align(o + 16 * (size_t)total_particles);
     w.bytes = o;
@@ -731,7 +723,8 @@ extern "C" int pyl_ma_batch_tiled(const pyl_batch_real *reals, int n_reals, cons
     if (n_items == 0) return PYL_OK;
     const unsigned grid = (unsigned)(num_sms() * BT_CTAS);
     const int split = bt_split(n_items);
-    bt_count_kernel<<<grid, BT_THREADS, 0, st>>>(reals, items, n_items, split, tile_base, ws.counts, ws.counters);
+    bt_count_kernel<<<grid, BT_THREADS, 0, st>>>(reals, items, n_items, split, tile_base, ws.counts, ws.adds,
+                                                 ws.counters);
     PYL_LAUNCH_CHECK();
     bt_scan_kernel<<<1, 1024, 0, st>>>(ws.counts, total_tiles, ws.offsets, ws.cursor);
     PYL_LAUNCH_CHECK();
@@ -741,16 +734,9 @@ extern "C" int pyl_ma_batch_tiled(const pyl_batch_real *reals, int n_reals, cons
     PYL_LAUNCH_CHECK();
     const unsigned max_parts = (unsigned)bt_max_parts(total_tiles), sms = (unsigned)num_sms();
     const size_t max_shared = bt_max_shared(total_tiles, total_particles);
-    const unsigned tb = (total_tiles + 255) / 256;
-    bt_adds_kernel<<<tb, 256, 0, st>>>(reals, n_reals, tile_base, total_tiles, ws.counts, ws.adds);
-    PYL_LAUNCH_CHECK();
-    bt_parts_kernel<<<tb, 256, 0, st>>>(reals, n_reals, tile_base, total_tiles, ws.counts, ws.adds, sms, ws.parts);
-    PYL_LAUNCH_CHECK();
-    bt_scan_kernel<<<1, 1024, 0, st>>>(ws.parts, total_tiles, ws.first_part, nullptr);
-    PYL_LAUNCH_CHECK();
-    bt_list_kernel<<<(total_tiles + 7) / 8, 256, 0, st>>>(
-        reals, n_reals, tile_base, total_tiles, ws.counts, ws.adds, sms, ws.first_part, max_parts,
-        (unsigned)max_shared, ws.counters + 3, ws.list);
+    bt_list_kernel<<<(total_tiles + 255) / 256, 256, 0, st>>>(reals, n_reals, tile_base, total_tiles, ws.counts, ws.adds,
+                                                              sms, max_parts, (unsigned)max_shared, ws.counters + 4,
+                                                              ws.counters + 3, ws.list);
     PYL_LAUNCH_CHECK();
     if (max_shared) {
         bt_share_zero_kernel<<<dim3(8, (unsigned)max_shared), 256, 0, st>>>(ws.counters + 3, ws.share);
@@ -758,7 +744,7 @@ extern "C" int pyl_ma_batch_tiled(const pyl_batch_real *reals, int n_reals, cons
     }
     PYL_CUDA(ensure_smem(bt_deposit_kernel, BT_DEPOSIT_SMEM));
     bt_deposit_kernel<<<sms, 1024, BT_DEPOSIT_SMEM, st>>>(
-        reals, tile_base, ws.list, ws.first_part + total_tiles, max_parts, ws.offsets, (unsigned)total_particles,
+        reals, tile_base, ws.list, ws.counters + 4, max_parts, ws.offsets, (unsigned)total_particles,
         ws.rec, ws.share, ws.done, ws.counters + 2);
     PYL_LAUNCH_CHECK();
     return PYL_OK;
