@@ -277,71 +277,41 @@ __device__ __forceinline__ int bt_real_of(const unsigned *__restrict__ tile_base
     return lo;
 }
 
-// The work list: a bin's parts of the plain grid, then of the interlaced one, bins in any
-// order (a warp reserves the places of its 32 bins).  Each grid's bin in parts takes a
-// BinShare.  With kernels of their own for the sum of additions, the parts of each bin and
-// their scan, four realizations of 512^3 took 27 us longer, one of 64^3 8.
-__global__ void __launch_bounds__(256) bt_list_kernel(const pyl_batch_real *__restrict__ reals, int n_reals,
-                                                      const unsigned *__restrict__ tile_base, unsigned total_tiles,
-                                                      const unsigned *__restrict__ counts,
-                                                      const unsigned long long *__restrict__ adds, unsigned sms,
-                                                      unsigned max_parts, unsigned max_shared, unsigned *n_parts,
-                                                      unsigned *shared_count, BtPart *__restrict__ list)
+// Parts of a bin of each grid of its realization, by the counts and the sum of additions.
+struct BtBin {
+    unsigned count, real, len, grids, parts;
+};
+
+__device__ __forceinline__ BtBin bt_bin(const pyl_batch_real *__restrict__ reals, int n_reals,
+                                        const unsigned *__restrict__ tile_base, unsigned total_tiles,
+                                        const unsigned *__restrict__ counts, unsigned long long adds, unsigned sms, unsigned t)
 {
-    const unsigned t = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31u;
-    unsigned count = 0u, real = 0u, len = 1u, grids = 1u, parts = 0u, shared = 0u;
-    if (t < total_tiles) {
-        count = counts[t];
-        real = (unsigned)bt_real_of(tile_base, n_reals, t);
-        len = bt_part_len(*adds, sms, reals[real].mas);
-        grids = reals[real].grid_interlaced ? 2u : 1u;
-        parts = count / len + (count % len != 0u);          // of each grid
-    }
-    unsigned end = parts * grids;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const unsigned v = __shfl_up_sync(0xffffffffu, end, o);
-        if (lane >= (unsigned)o) end += v;
-    }
-    const unsigned total = __shfl_sync(0xffffffffu, end, 31);
-    if (total == 0u) return;
-    unsigned first = 0u;
-    if (lane == 0u) first = atomicAdd(n_parts, total);
-    first = __shfl_sync(0xffffffffu, first, 0) + end - parts * grids;
-    if (parts > 1u) shared = atomicAdd(shared_count, grids);
-    // no BinShare left (bt_max_shared has one for every bin in parts, unless the items hold more
-    // particles than the caller's total): whole bins, the other parts empty
-    const bool whole = parts > 1u && shared + grids > max_shared;
-    auto entry = [&](unsigned i, unsigned tile, unsigned r, unsigned n, unsigned l, unsigned per_grid, unsigned sh, bool w) {
-        const unsigned from = (i % per_grid) * l, g = i / per_grid;
-        return w ? BtPart{tile, r, 0u, from ? 0u : n, g, 1u, 0u, 0u} : BtPart{tile, r, from, min(l, n - from), g, per_grid, sh + g, 0u};
-    };
-    if (parts == 1u)
-        for (unsigned i = 0; i < grids && first + i < max_parts; i++) list[first + i] = entry(i, t, real, count, len, 1u, 0u, false);
-    for (unsigned many = __ballot_sync(0xffffffffu, parts > 1u); many; many &= many - 1u) {
-        const int s = __ffs(many) - 1;                       // bins in parts: a warp for each
-        const unsigned b = __shfl_sync(0xffffffffu, first, s), p = __shfl_sync(0xffffffffu, parts, s);
-        const unsigned n = __shfl_sync(0xffffffffu, p * grids, s), r = __shfl_sync(0xffffffffu, real, s);
-        const unsigned c = __shfl_sync(0xffffffffu, count, s), l = __shfl_sync(0xffffffffu, len, s);
-        const unsigned sh = __shfl_sync(0xffffffffu, shared, s), tile = __shfl_sync(0xffffffffu, t, s);
-        const bool w = __shfl_sync(0xffffffffu, (int)whole, s) != 0;
-        for (unsigned i = lane; i < n && b + i < max_parts; i += 32) list[b + i] = entry(i, tile, r, c, l, p, sh, w);
-    }
+    if (t >= total_tiles) return BtBin{0u, 0u, 1u, 1u, 0u};
+    const unsigned c = counts[t], real = (unsigned)bt_real_of(tile_base, n_reals, t);
+    const unsigned len = bt_part_len(adds, sms, reals[real].mas);
+    return BtBin{c, real, len, reals[real].grid_interlaced ? 2u : 1u, c / len + (c % len != 0u)};
 }
 
-// Zeroes the words of the BinShares in use (blockIdx.y), gridDim.x CTAs each.
-__global__ void __launch_bounds__(256) bt_share_zero_kernel(const unsigned *__restrict__ shared_count,
-                                                            unsigned long long *__restrict__ share)
+// CTA 0: exclusive scan of n counts into offsets[0..n] and cursor[0..n).  CTA b > 0: the
+// list entries of its 1024 bins, into entries[b - 1].
+__global__ void __launch_bounds__(1024) bt_scan_kernel(const pyl_batch_real *__restrict__ reals, int n_reals,
+                                                       const unsigned *__restrict__ tile_base,
+                                                       const unsigned *__restrict__ counts, unsigned n,
+                                                       const unsigned long long *__restrict__ adds, unsigned sms,
+                                                       unsigned *__restrict__ offsets, unsigned *__restrict__ cursor,
+                                                       unsigned *__restrict__ entries)
 {
-    if (blockIdx.y >= *shared_count) return;
-    unsigned long long *z = share + blockIdx.y * BT_SHARE_CELLS;
-    for (size_t i = blockIdx.x * blockDim.x + threadIdx.x; i < BT_SHARE_CELLS; i += gridDim.x * blockDim.x) z[i] = 0ull;
-}
-
-// Exclusive scan of n counts into offsets[0..n] and cursor[0..n), one CTA.
-__global__ void __launch_bounds__(1024) bt_scan_kernel(const unsigned *__restrict__ counts, unsigned n,
-                                                       unsigned *__restrict__ offsets, unsigned *__restrict__ cursor)
-{
+    if (blockIdx.x) {
+        __shared__ unsigned sum;
+        if (threadIdx.x == 0) sum = 0u;
+        __syncthreads();
+        const BtBin b = bt_bin(reals, n_reals, tile_base, n, counts, *adds, sms, (blockIdx.x - 1) * 1024 + threadIdx.x);
+        const unsigned w = __reduce_add_sync(0xffffffffu, b.parts * b.grids);
+        if ((threadIdx.x & 31) == 0 && w) atomicAdd(&sum, w);
+        __syncthreads();
+        if (threadIdx.x == 0) entries[blockIdx.x - 1] = sum;
+        return;
+    }
     __shared__ unsigned long long part[1024];
     const unsigned per = (n + blockDim.x - 1) / blockDim.x;
     const unsigned b = threadIdx.x * per, e = min(n, b + per);
@@ -362,6 +332,71 @@ __global__ void __launch_bounds__(1024) bt_scan_kernel(const unsigned *__restric
         run += counts[i];
     }
     if (threadIdx.x == blockDim.x - 1) offsets[n] = (unsigned)part[threadIdx.x];
+}
+
+// The work list, in bin order: a bin's parts of the plain grid, then of the interlaced one.
+// Each grid's bin in parts takes a BinShare.  (In any order, 24 realizations took 2 % longer:
+// neighbouring bins add to the same cells.)  With kernels of their own for the sum of
+// additions, the parts of each bin and their scan, four realizations of 512^3 took 27 us
+// longer, one of 64^3 8.
+__global__ void __launch_bounds__(1024) bt_list_kernel(const pyl_batch_real *__restrict__ reals, int n_reals,
+                                                       const unsigned *__restrict__ tile_base, unsigned total_tiles,
+                                                       const unsigned *__restrict__ counts,
+                                                       const unsigned long long *__restrict__ adds, unsigned sms,
+                                                       const unsigned *__restrict__ entries, unsigned max_parts,
+                                                       unsigned max_shared, unsigned *n_parts, unsigned *shared_count,
+                                                       BtPart *__restrict__ list)
+{
+    __shared__ unsigned before, warps[32];
+    const unsigned t = blockIdx.x * 1024 + threadIdx.x, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    if (threadIdx.x == 0) before = 0u;
+    __syncthreads();
+    unsigned sum = 0u;
+    for (unsigned i = threadIdx.x; i < blockIdx.x; i += 1024) sum += entries[i];
+    if (sum) atomicAdd(&before, sum);
+    const BtBin bin = bt_bin(reals, n_reals, tile_base, total_tiles, counts, *adds, sms, t);
+    const unsigned mine = bin.parts * bin.grids;
+    unsigned end = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned v = __shfl_up_sync(0xffffffffu, end, o);
+        if (lane >= (unsigned)o) end += v;
+    }
+    if (lane == 31u) warps[warp] = end;
+    __syncthreads();
+    unsigned first = before + end - mine;
+    for (unsigned w = 0; w < warp; w++) first += warps[w];
+    if (threadIdx.x == 1023u && blockIdx.x + 1 == gridDim.x) *n_parts = first + mine;
+    unsigned shared = 0u;
+    if (bin.parts > 1u) shared = atomicAdd(shared_count, bin.grids);
+    // no BinShare left (bt_max_shared has one for every bin in parts, unless the items hold more
+    // particles than the caller's total): whole bins, the other parts empty
+    const bool whole = bin.parts > 1u && shared + bin.grids > max_shared;
+    if (bin.parts == 1u)
+        for (unsigned g = 0; g < bin.grids && first + g < max_parts; g++)
+            list[first + g] = BtPart{t, bin.real, 0u, bin.count, g, 1u, 0u, 0u};
+    for (unsigned many = __ballot_sync(0xffffffffu, bin.parts > 1u); many; many &= many - 1u) {
+        const int s = __ffs(many) - 1;                       // bins in parts: a warp for each
+        const unsigned b = __shfl_sync(0xffffffffu, first, s), p = __shfl_sync(0xffffffffu, bin.parts, s);
+        const unsigned n = __shfl_sync(0xffffffffu, mine, s), r = __shfl_sync(0xffffffffu, bin.real, s);
+        const unsigned c = __shfl_sync(0xffffffffu, bin.count, s), l = __shfl_sync(0xffffffffu, bin.len, s);
+        const unsigned sh = __shfl_sync(0xffffffffu, shared, s), tile = __shfl_sync(0xffffffffu, t, s);
+        const unsigned w = __shfl_sync(0xffffffffu, whole ? 1u : 0u, s);
+        for (unsigned i = lane; i < n && b + i < max_parts; i += 32) {
+            const unsigned from = (i % p) * l, g = i / p;
+            list[b + i] = w ? BtPart{tile, r, 0u, from ? 0u : c, g, 1u, 0u, 0u}
+                            : BtPart{tile, r, from, min(l, c - from), g, p, sh + g, 0u};
+        }
+    }
+}
+
+// Zeroes the words of the BinShares in use (blockIdx.y), gridDim.x CTAs each.
+__global__ void __launch_bounds__(256) bt_share_zero_kernel(const unsigned *__restrict__ shared_count,
+                                                            unsigned long long *__restrict__ share)
+{
+    if (blockIdx.y >= *shared_count) return;
+    unsigned long long *z = share + blockIdx.y * BT_SHARE_CELLS;
+    for (size_t i = blockIdx.x * blockDim.x + threadIdx.x; i < BT_SHARE_CELLS; i += gridDim.x * blockDim.x) z[i] = 0ull;
 }
 
 // Exclusive scan of v[0..n) in place (each thread n / blockDim.x consecutive entries);
@@ -624,7 +659,7 @@ __global__ void __launch_bounds__(1024) bt_deposit_kernel(const pyl_batch_real *
 }
 
 struct BtWs {
-    unsigned *counts, *offsets, *cursor, *counters, *done;
+    unsigned *counts, *offsets, *cursor, *counters, *done, *entries;
     unsigned long long *adds, *share;
     BtPart *list;
     float4 *rec;
@@ -650,6 +685,7 @@ BtWs bt_layout(void *base, unsigned total_tiles, long long total_particles)
     w.zero_bytes = 32 + 4 * shared;
     o = bt_align(o + w.zero_bytes);
     w.share = (unsigned long long *)(b + o); o = bt_align(o + 8 * BT_SHARE_CELLS * shared);
+    w.entries = (unsigned *)(b + o); o = bt_align(o + 4 * (((size_t)total_tiles + 1023) / 1024));
     w.list = (BtPart *)(b + o); o = bt_align(o + sizeof(BtPart) * bt_max_parts(total_tiles));
     w.rec = (float4 *)(b + o); o = bt_align(o + 16 * (size_t)total_particles);
     w.bytes = o;
@@ -726,17 +762,18 @@ extern "C" int pyl_ma_batch_tiled(const pyl_batch_real *reals, int n_reals, cons
     bt_count_kernel<<<grid, BT_THREADS, 0, st>>>(reals, items, n_items, split, tile_base, ws.counts, ws.adds,
                                                  ws.counters);
     PYL_LAUNCH_CHECK();
-    bt_scan_kernel<<<1, 1024, 0, st>>>(ws.counts, total_tiles, ws.offsets, ws.cursor);
+    const unsigned sms = (unsigned)num_sms(), groups = total_tiles / 1024 + (total_tiles % 1024 != 0);
+    bt_scan_kernel<<<1 + groups, 1024, 0, st>>>(reals, n_reals, tile_base, ws.counts, total_tiles, ws.adds, sms, ws.offsets,
+                                                ws.cursor, ws.entries);
     PYL_LAUNCH_CHECK();
     PYL_CUDA(ensure_smem(bt_place_kernel, BT_PLACE_SMEM));
     bt_place_kernel<<<grid, BT_THREADS, BT_PLACE_SMEM, st>>>(reals, items, n_items, split, tile_base, ws.cursor,
                                                        (unsigned)total_particles, ws.rec, ws.counters + 1);
     PYL_LAUNCH_CHECK();
-    const unsigned max_parts = (unsigned)bt_max_parts(total_tiles), sms = (unsigned)num_sms();
+    const unsigned max_parts = (unsigned)bt_max_parts(total_tiles);
     const size_t max_shared = bt_max_shared(total_tiles, total_particles);
-    bt_list_kernel<<<(total_tiles + 255) / 256, 256, 0, st>>>(reals, n_reals, tile_base, total_tiles, ws.counts, ws.adds,
-                                                              sms, max_parts, (unsigned)max_shared, ws.counters + 4,
-                                                              ws.counters + 3, ws.list);
+    bt_list_kernel<<<groups, 1024, 0, st>>>(reals, n_reals, tile_base, total_tiles, ws.counts, ws.adds, sms, ws.entries,
+                                            max_parts, (unsigned)max_shared, ws.counters + 4, ws.counters + 3, ws.list);
     PYL_LAUNCH_CHECK();
     if (max_shared) {
         bt_share_zero_kernel<<<dim3(8, (unsigned)max_shared), 256, 0, st>>>(ws.counters + 3, ws.share);
