@@ -233,7 +233,9 @@ __global__ void __launch_bounds__(BT_THREADS, BT_CTAS) bt_count_kernel(const pyl
 }
 
 // Parts of a batch of `adds` corner additions: at most BT_PARTS_PER_SM an SM, none below
-// PART_ADDS.
+// PART_ADDS.  Bins of less than two PART_ADDS stay whole: their longer part takes as long,
+// and the words come on top (100 realizations of 20,000 particles on 32^3, PCS interlaced: 425
+// us in parts, 368 whole, 383 before bins were divided).
 constexpr unsigned BT_PARTS_PER_SM = 4;
 
 __device__ __forceinline__ unsigned bt_part_len(unsigned long long adds, unsigned sms, int mas)
@@ -289,7 +291,8 @@ __device__ __forceinline__ BtBin bt_bin(const pyl_batch_real *__restrict__ reals
     if (t >= total_tiles) return BtBin{0u, 0u, 1u, 1u, 0u};
     const unsigned c = counts[t], real = (unsigned)bt_real_of(tile_base, n_reals, t);
     const unsigned len = bt_part_len(adds, sms, reals[real].mas);
-    return BtBin{c, real, len, reals[real].grid_interlaced ? 2u : 1u, c / len + (c % len != 0u)};
+    const bool whole = (unsigned long long)c * bt_corners(reals[real].mas) < 2 * PART_ADDS;
+    return BtBin{c, real, len, reals[real].grid_interlaced ? 2u : 1u, whole ? (c != 0u) : c / len + (c % len != 0u)};
 }
 
 // CTA 0: exclusive scan of n counts into offsets[0..n] and cursor[0..n).  CTA b > 0: the
