@@ -800,10 +800,11 @@ int sorted_pass(const float *pos, const float *w, long long n, float *out, int d
     } else {
         constexpr int H = MAS - 1;
         // layers per CTA: SD_CTA_LAYERS, or fewer (each CTA brings its own S-1 halo layers)
-        // until the CTAs are two per SM
+        // until the CTAs are two per SM, below eight until they are one: a thread's walk is as
+        // long as its layers (2^20 particles on 32^3, CIC, eight 221 us, two 138)
         const unsigned gy = (unsigned)((dims + SDY - H - 1) / (SDY - H)), gx = (unsigned)((dims + SDX - H - 1) / (SDX - H));
         int zs = SD_CTA_LAYERS;
-        while (zs > 8 && (long long)gx * gy * ((dims + zs - 1) / zs) < 2LL * num_sms()) zs /= 2;
+        while (zs > 2 && (long long)gx * gy * ((dims + zs - 1) / zs) < (zs > 8 ? 2LL : 1LL) * num_sms()) zs /= 2;
         constexpr size_t smem = SdShape<MAS>::SMEM;
         const SdCrowd crowd = sd_crowd_layout(spos == ws.rec[0] ? ws.rec[1] : ws.rec[0], n);
         if (crowd.at) {

@@ -170,3 +170,10 @@ def test_crowded_cells_cost_little(MASL, mas, dims):
     one: 6 to 141 times the time of as many all over the box)."""
     n = 1 << 24
     assert time_us(MASL, uniform(n, part=0.05), dims, mas) <= 4.0 * time_us(MASL, uniform(n), dims, mas)
+
+
+def test_small_grids_keep_short_walks(MASL):
+    """2^20 particles on 32^3 (32 a cell) in little more than the time of 64^3 (1.45 times
+    with eight layers a CTA)."""
+    pos = uniform(1 << 20)
+    assert time_us(MASL, pos, 32, 'CIC') <= 1.2 * time_us(MASL, pos, 64, 'CIC')
