@@ -176,7 +176,7 @@ inline size_t owned_halo_floats(int mas, int dims, bool inter)
 
 // Parts of a bin's records.  Grids of fewer bins than half the SMs leave most of the chip
 // idle when a CTA takes a whole bin: its records then go to several CTAs, which add
-// their cells to 64-bit fixed-point words of the grid.  A part is an eighth of an SM's
+// their cells to 64-bit fixed-point words of the bin.  A part is an eighth of an SM's
 // share of all records, and at least PART_ADDS corner additions, with four times the
 // parts of an average bin for the heavier ones (the last part takes what is left).  An
 // average bin of less than two parts stays whole: its longest part takes as long, and the
@@ -202,11 +202,12 @@ inline BinParts bin_parts(long long n, int mas, int dims, bool inter)
     return BinParts{(unsigned)len, (unsigned)std::min(4 * (n / bins / len + 1), 65535LL)};
 }
 
-// Bytes of the fixed-point words of the grids (0: whole bins).
+// Bytes of the fixed-point words of the bins' cells, halo included (0: whole bins).
 inline size_t bin_share_bytes(long long n, int mas, int dims, bool inter)
 {
     if (bin_parts(n, mas, dims, inter).parts == 1) return 0;
-    return sizeof(unsigned long long) * (size_t)dims * dims * dims * (inter ? 2 : 1);
+    const size_t nt = (size_t)((dims + TB - 1) / TB), e = TB + (mas == PYL_MAS_NGP ? 0 : mas - 1) + (inter ? 1 : 0);
+    return sizeof(unsigned long long) * nt * nt * nt * e * e * e * (inter ? 2 : 1);
 }
 
 // Bytes behind the records of a tiled workspace: the owned-cell halo blocks, or the words

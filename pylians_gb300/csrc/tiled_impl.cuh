@@ -1227,49 +1227,55 @@ __device__ __forceinline__ void fx_write_out(const unsigned *smw, float *out, co
     }
 }
 
-// Write-out of a bin's part (BinParts): the cells' sums are added to the grid's 64-bit
+// Write-out of a bin's part (BinParts): the cells' sums are added to the bin's 64-bit
 // fixed-point words, so the words do not depend on how the records were divided or in
-// which order the parts end; share_finish_kernel adds them to the grid.  The sums of a part
-// redone in float32 (a cell of 512 or more) go there in the same units, and what is
-// smaller than a unit to the grid itself, so that small cells keep their 24 bits; float
-// sums of weights (any magnitude) and what is not finite go to the grid.
+// which order the parts end; share_finish_kernel adds them to the grid as one CTA would
+// have added the bin's cells, with its roundings (words of the grid's cells, which all bins
+// add to, would round a cell once instead of once for each bin).  The sums of a part redone in float32 (a cell
+// of 512 or more) go there in the same units, and what is smaller than a unit to the grid
+// itself, so that small cells keep their 24 bits; float sums of weights (any magnitude) and
+// what is not finite go to the grid.
 template <int MAS, bool INTER, bool FLOAT>
 __device__ __forceinline__ void fx_share_out(const unsigned *smw, unsigned long long *share, float *out, const int *o,
                                              int dims, bool interior, float scale, bool weighted)
 {
     constexpr float UNITS = MAS == PYL_MAS_NGP ? 1.0f : FX_SCALE;   // of 1 (NGP: counts)
+    if (!FLOAT) {
+        for (int c = threadIdx.x; c < FxShape<MAS, INTER>::CELLS; c += 1024)
+            if (smw[c] != 0u) atomicAdd(share + c, (unsigned long long)smw[c]);
+        return;
+    }
     fx_each_cell<MAS, INTER>([&](long long i, int c) {
-        const unsigned w = smw[c];
-        if (w == 0u) return;
-        if (!FLOAT) {
-            atomicAdd(share + i, (unsigned long long)w);
+        const float v = __uint_as_float(smw[c]);
+        if (v == 0.0f) return;
+        if (!weighted && fabsf(v) < 1e12f) {
+            const long long u = __float2ll_rn(__fmul_rn(v, UNITS));
+            const float rest = __fsub_rn(v, __fmul_rn(__ll2float_rn(u), 1.0f / UNITS));  // exact; 0 from 2 on
+            if (u) atomicAdd(share + c, (unsigned long long)u);
+            if (rest != 0.0f) atomicAdd(out + i, __fmul_rn(rest, scale));
         } else {
-            const float v = __uint_as_float(w);
-            if (!weighted && fabsf(v) < 1e12f) {
-                const long long u = __float2ll_rn(__fmul_rn(v, UNITS));
-                const float rest = __fsub_rn(v, __fmul_rn(__ll2float_rn(u), 1.0f / UNITS));  // exact; 0 from 2 on
-                if (u) atomicAdd(share + i, (unsigned long long)u);
-                if (rest != 0.0f) atomicAdd(out + i, __fmul_rn(rest, scale));
-            } else {
-                atomicAdd(out + i, __fmul_rn(v, scale));
-            }
+            atomicAdd(out + i, __fmul_rn(v, scale));
         }
     }, o, dims, interior);
 }
 
-// grid += the words' values (NGP: counts, or fixed-point weights whose unit is in scale).
-template <int MAS>
-__global__ void __launch_bounds__(256) share_finish_kernel(const unsigned long long *__restrict__ share, long long n,
-                                                           OutScale sc, float *__restrict__ grid, const unsigned *err)
+// The words' values (NGP: counts, or fixed-point weights whose unit is in scale) of bin
+// blockIdx.x, gridDim.y CTAs each, into the grid.
+template <int MAS, bool INTER>
+__global__ void __launch_bounds__(1024) share_finish_kernel(const unsigned long long *__restrict__ share, int nt, int dims,
+                                                            OutScale sc, float *__restrict__ grid, const unsigned *err)
 {
     if (*(const volatile unsigned *)err) return;        // the deposit left (some of) its bins out
+    constexpr int E = FxShape<MAS, INTER>::E, CELLS = FxShape<MAS, INTER>::CELLS;
     const float scale = out_scale(sc);
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-        const long long w = (long long)share[i];
+    const int b = blockIdx.x, tx = b / (nt * nt), ty = b / nt % nt, tz = b % nt;
+    const long long d = dims;
+    for (int c = blockIdx.y * 1024 + threadIdx.x; c < CELLS; c += gridDim.y * 1024) {
+        const long long w = (long long)share[(size_t)b * CELLS + c];
         if (w == 0) continue;
+        const long long gx = add_wrap(tx * TB, c / (E * E), d), gy = add_wrap(ty * TB, c / E % E, d), gz = add_wrap(tz * TB, c % E, d);
         const float v = __ll2float_rn(w);
-        grid[i] = __fadd_rn(grid[i], __fmul_rn(MAS == PYL_MAS_NGP ? v : __fmul_rn(v, FX_INV), scale));
+        atomicAdd(grid + (gx * d + gy) * d + gz, __fmul_rn(MAS == PYL_MAS_NGP ? v : __fmul_rn(v, FX_INV), scale));
     }
 }
 
@@ -1460,7 +1466,7 @@ __device__ __forceinline__ bool fx_grid(const FxStage &sg, unsigned &q0, float i
 
 // PARTS: a CTA takes `part` records of a bin (BinParts), CTA blockIdx.y those from
 // blockIdx.y * part on and the last one all that are left, and adds its cells to the
-// words `share` of the grids (fx_share_out), the plain grid's first.  (A kernel of its
+// words `share` of the bins (fx_share_out), the plain grid's first.  (A kernel of its
 // own: the 512^3 interlaced PCS deposit ran 3% slower with both in one.)
 template <int MAS, bool INTER, int R, bool P2, bool TOT, bool FREE, bool PARTS = false>
 __global__ void __launch_bounds__(1024) bin_deposit_fx_tma_kernel(
@@ -1515,15 +1521,16 @@ __global__ void __launch_bounds__(1024) bin_deposit_fx_tma_kernel(
         sg.inv_w = inv_w;
         sg.use_float = inv_w ? reinterpret_cast<const int *>(inv_w + 2) : nullptr;
         sg.err = err;
+        const size_t bin = PARTS ? ((size_t)tx * g.nt + ty) * g.nt + tz : 0;
         float *hb = ow.on && HC > 0 ? ow.halo + tile * HC : nullptr;
         const float *prev = have_prev && hb ? hb - HC : nullptr;
         if (!fx_grid<MAS, INTER, R, 0, P2, TOT, FREE, PARTS>(sg, q0, inv, halfcell, dims, o, smw, grid, interior, scale, ow, hb,
-                                                             prev, share))
+                                                             prev, PARTS ? share + bin * FS::CELLS : nullptr))
             return;
         if (INTER &&
             !fx_grid<MAS, INTER, R, 1, P2, TOT, FREE, PARTS>(sg, q0, inv, halfcell, dims, o, smw, grid2, interior, scale, ow,
                                        hb ? hb + ow.stride : nullptr, prev ? prev + ow.stride : nullptr,
-                                       PARTS ? share + (size_t)dims * dims * dims : nullptr))
+                                       PARTS ? share + ((size_t)g.nt * g.nt * g.nt + bin) * FS::CELLS : nullptr))
             return;
         have_prev = true;
     }
@@ -1579,10 +1586,10 @@ int launch_deposit_fx(const TiledWs &ws, TileGeom g, float inv, float halfcell, 
                                                        inv_w, err, bp.len, share);
         PYL_LAUNCH_CHECK();
         if (share) {
-            const long long cells = (long long)g.dims * g.dims * g.dims;
+            const int bins = g.nt * g.nt * g.nt;
             for (int k = 0; k < (I ? 2 : 1); k++) {
-                share_finish_kernel<MAS><<<grid_blocks(cells, 256), 256, 0, st>>>(share + k * cells, cells, sc,
-                                                                                  k ? grid2 : grid, err);
+                share_finish_kernel<MAS, I><<<dim3(bins, 8), 1024, 0, st>>>(share + (size_t)k * bins * FS::CELLS, g.nt, g.dims,
+                                                                            sc, k ? grid2 : grid, err);
                 PYL_LAUNCH_CHECK();
             }
         }

@@ -182,3 +182,36 @@ def test_average_bins_of_less_than_two_parts_stay_whole(mods, dims, mas, inter, 
     words = 8 * dims ** 3 * (2 if inter else 1)
     assert size(n, 3, dims, mas, 2, inter) - size(n - bins, 3, dims, mas, 2, inter) >= words
     assert size(n - bins, 3, dims, mas, 2, inter) - size(n - 2 * bins, 3, dims, mas, 2, inter) < words // 4
+
+
+@pytest.mark.parametrize('dims', [64, 114])
+@pytest.mark.parametrize('mas,inter', [('CIC', 0), ('TSC', 1), ('PCS', 0)])
+def test_parts_round_cells_as_whole_bins_do(mods, dims, mas, inter):
+    """The same deposit with a workspace that has no room for the words (whole bins): the
+    same bits in every cell that one or two bins add to (three and more meet in any order)."""
+    from pylians_gb300 import _lib
+    from pylians_gb300._device import ptr, stream_ptr
+    s = {'CIC': 2, 'TSC': 3, 'PCS': 4}[mas]
+    bins = (-(-dims // 32)) ** 3
+    n = int(3 * bins * (1 << 20) / (s ** 3 * (1 + inter)))
+    g = torch.Generator(device='cuda')
+    g.manual_seed(dims)
+    pos = torch.rand((n, 3), generator=g, device='cuda') * (BOX * 0.999)
+    size = _lib.load().pyl_ma_workspace_size(n, 3, dims, s, 2, inter)
+    words = 8 * bins * (32 + s - 1 + inter) ** 3 * (1 + inter)
+    out = []
+    for nbytes in (size, size - words):
+        ws = torch.empty(nbytes, dtype=torch.uint8, device='cuda')
+        grids = torch.zeros((1 + inter, dims, dims, dims), device='cuda')
+        _lib.call('pyl_ma', ptr(pos), None, n, 3, ptr(grids[0]), ptr(grids[1]) if inter else None, dims, BOX, s, 2, 0, ptr(ws),
+                  nbytes, stream_ptr())
+        out.append(grids.cpu().numpy())
+    k = np.arange(dims)
+    halo = k % 32 < s - 1 + inter
+    if dims % 32:                            # the last bin is cut off: its halo wraps onto more
+        halo |= k % 32 < (s - 1 + inter + 32 - dims % 32)
+    h = halo[:, None, None].astype(int) + halo[None, :, None] + halo[None, None, :]
+    cells = h <= 1
+    assert cells.mean() > 0.3
+    for i in range(1 + inter):
+        assert np.array_equal(out[0][i][cells], out[1][i][cells])
