@@ -172,7 +172,9 @@ int pyl_scale(float *p, int64_t n, float factor, void *stream);
  * realization's MAS and interlacing), adding scale * deposit into the grids
  * (pre-filled by the caller, e.g. with -1 for the overdensity).  reals, items
  * and tile_base live in device memory; total_particles = sum of item counts.
- * ctas_per_sm (1..8) is checked; every launch here has its own grid. */
+ * ctas_per_sm (1..8) is checked; every launch here has its own grid.  The workspace holds
+ * 16 bytes a particle, a few words a bin, and 373 KB for each bin that may be divided:
+ * at most 4 an SM, none below 2^20 corner additions (16384 PCS particles). */
 size_t pyl_ma_batch_tiled_workspace_size(uint32_t total_tiles, int64_t total_particles);
 int pyl_ma_batch_tiled(const pyl_batch_real *reals, int n_reals, const pyl_batch_item *items, int n_items,
                        const uint32_t *tile_base, uint32_t total_tiles, int64_t total_particles, void *workspace,
@@ -448,8 +450,9 @@ int pyl_wait_probe(unsigned arm_bytes, long long cycles, unsigned *completed, vo
  * eight terms added in the reference's order; indices wrap non-negatively.
  * pyl_cic_interp_slabs gives the same bits from a workspace of
  * pyl_cic_interp_workspace_size() bytes (16-byte aligned), faster for many particles
- * in no order on a grid larger than L2; the size is 0 where pyl_cic_interp is the
- * faster one whatever the order.
+ * in no order on a grid larger than L2; the size (18 bytes a particle of at most
+ * 2^25, and run starts: up to 0.7 GB) is 0 where pyl_cic_interp is the faster one
+ * whatever the order.
  * pyl_pos_redshift_space replaces redshift_space_library.pos_redshift_space
  * (library/redshift_space_library.pyx:29-43): pos[:,axis] += vel[:,axis] *
  * (1+redshift)/Hubble in place, then positions above box_size or below 0 become

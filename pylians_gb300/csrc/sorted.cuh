@@ -10,8 +10,8 @@ namespace pyl {
 // dims^3 <= 2^32 cells and fewer than 2^32 particles.
 bool sorted_supported(long long n, int dims);
 
-// Workspace bytes of the sorted strategy (keys, values, digit histograms,
-// per-cell runs, positions in sorted order).
+// Workspace bytes of the sorted strategy (records twice, digit histograms, column
+// starts and empty stretches).
 size_t sorted_workspace_bytes(long long n, int dims);
 
 // Deposits n particles into grid (and the half-cell-shifted grid2 when non-null).
